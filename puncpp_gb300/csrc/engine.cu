@@ -1092,15 +1092,26 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
         (rc = upload(s, &d_dofs, dof32)) || (rc = upload(s, &d_dvinv, h.dv_inv)) || (rc = dalloc(s, &d_E, 4 * h.nc)))
         return bail(rc);
     cudaMemset(d_E, 0, sizeof(double) * 4 * h.nc);
-    if (cfg.precision == PG_MIXED) {
+    {
         float4 *cf;
+        float *d_abs;
+        if ((rc = dalloc(s, &cf, 4 * h.nc)) || (rc = dalloc(s, &d_abs, 1))) return bail(rc);
+        // points of a step stay within a few domain sizes of the origin
+        double X = 0.0;
+        for (int j = 0; j < 3; ++j)
+            X = std::max(X, std::max(std::fabs(h.bbox_lo[j]), std::fabs(h.bbox_hi[j])) + h.bbox_hi[j] - h.bbox_lo[j]);
+        launch_float_tables(d_bary, d_planes, reinterpret_cast<const int4 *>(d_nbr), (int32_t)h.nc, 4.0 * X, cf, d_abs,
+                            s->stream);
+        if (cudaMemcpyAsync(&s->dm.lam_abs, d_abs, sizeof(float), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
+            cudaStreamSynchronize(s->stream) != cudaSuccess)
+            return bail(fail(PG_ERR_CUDA, "pg_create: cell records"));
+        s->dm.cell_f = cf;
+    }
+    if (cfg.precision == PG_MIXED) {
         float *ef;
-        if ((rc = dalloc(s, &cf, 4 * h.nc)) || (rc = dalloc(s, &ef, 4 * h.nc)) || (rc = dalloc(s, &s->rho_fixed, h.ndof)))
-            return bail(rc);
+        if ((rc = dalloc(s, &ef, 4 * h.nc)) || (rc = dalloc(s, &s->rho_fixed, h.ndof))) return bail(rc);
         cudaMemset(ef, 0, sizeof(float) * 4 * h.nc);
         cudaMemset(s->rho_fixed, 0, sizeof(unsigned long long) * h.ndof);
-        launch_float_tables(d_bary, reinterpret_cast<const int4 *>(d_nbr), (int32_t)h.nc, cf, s->stream);
-        s->dm.cell_f = cf;
         s->dm.E_f = ef;
     } else if (cfg.precision != PG_FP64) {
         return bail(fail(PG_ERR_ARG, "pg_create: unknown precision"));
@@ -1119,6 +1130,17 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
     if ((rc = upload(s, &d_binptr, h.bin_ptr)) || (rc = upload(s, &d_bincells, h.bin_cells))) return bail(rc);
     s->dm.bin_ptr = d_binptr;
     s->dm.bin_cells = d_bincells;
+    {
+        // the cells fill the bounding box (a convex domain without a hole)
+        double vol = 0.0, box = 1.0;
+        for (double v : h.volume) vol += v;
+        for (int j = 0; j < 3; ++j) {
+            box *= h.bbox_hi[j] - h.bbox_lo[j];
+            s->dm.lo_f[j] = (float)h.bbox_lo[j];
+            s->dm.bin_inv_f[j] = (float)(1.0 / h.bin_h[j]);
+        }
+        s->dm.box = std::fabs(vol - box) <= 1e-9 * box && cfg.max_walk_steps >= kBoxWalkLimit ? 1 : 0;
+    }
 
     // fields
     if ((rc = dalloc(s, &s->rho_acc, h.ndof)) || (rc = dalloc(s, &s->rho, h.ndof)) || (rc = dalloc(s, &s->phi, h.ndof)) ||

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_inject_generate(DevMesh m, DevP
         z = z + r * ip.dt * vz;
         p.x[i] = x; p.y[i] = y; p.z[i] = z;
         p.vx[i] = vx; p.vy[i] = vy; p.vz[i] = vz;
-        const int c = walk_fp64(m, x, y, z, (int)F[13], max_steps);
+        const int c = walk_fp64<false>(m, x, y, z, (int)F[13], max_steps);
         if (c == kWalkFail) { raise_device_error(st, PG_ERR_WALK_LIMIT, i); p.cell[i] = kDead; continue; }
         if (c < 0) { p.cell[i] = kDead; continue; }
         p.cell[i] = c;

@@ -61,15 +61,6 @@ __device__ __forceinline__ void deposit_lambdas(bool agg, int c, const float l[4
     atomicAdd(rho_fixed + d.w, (unsigned long long)v3);
 }
 
-// Cell record of c: barycentric rows 0-2 and the neighbours (int bits).
-struct CellRec {
-    float4 r0, r1, r2, nb;
-};
-__device__ __forceinline__ CellRec load_rec(const DevMesh &m, int c) {
-    const float4 *R = m.cell_f + 4 * (size_t)c;
-    return CellRec{__ldg(R), __ldg(R + 1), __ldg(R + 2), __ldg(R + 3)};
-}
-
 template <bool PUSH, bool HAS_B, bool ACCEL, bool MOVE, bool PERIODIC, bool WALK, bool DEPOSIT>
 __global__ void __launch_bounds__(512, 2) k_mixed(DevMesh m, DevParticles p, int64_t n_slots, MixedParams mp,
                                                    int max_steps, unsigned long long *__restrict__ rho_fixed,
@@ -145,32 +136,19 @@ __global__ void __launch_bounds__(512, 2) k_mixed(DevMesh m, DevParticles p, int
             if (MOVE) {
                 x = fmaf(mp.dt, vx, x); y = fmaf(mp.dt, vy, y); z = fmaf(mp.dt, vz, z);
                 if (PERIODIC) {
-                    x -= mp.Ld[0] * floorf(x / mp.Ld[0]);
-                    y -= mp.Ld[1] * floorf(y / mp.Ld[1]);
-                    z -= mp.Ld[2] * floorf(z / mp.Ld[2]);
+                    // 0 < x < L: the floor is 0
+                    if (!(x > 0.0f && x < mp.Ld[0])) x -= mp.Ld[0] * floorf(x / mp.Ld[0]);
+                    if (!(y > 0.0f && y < mp.Ld[1])) y -= mp.Ld[1] * floorf(y / mp.Ld[1]);
+                    if (!(z > 0.0f && z < mp.Ld[2])) z -= mp.Ld[2] * floorf(z / mp.Ld[2]);
                 }
                 p.xf[i] = x; p.yf[i] = y; p.zf[i] = z;
             }
         }
         float l[4];
         if (WALK) {
-            // walk_mixed with the first cell's record already loaded; the
-            // last cell's lambdas are the deposit's
-            float e[4];
-            int cc = c, end = kWalkFail;
-            for (int it = 0; it < max_steps; ++it) {
-                if (!have_rec) R = load_rec(m, cc);
-                have_rec = false;
-                lambdas_f32(R.r0, R.r1, R.r2, x, y, z, l, e);
-                int next;
-                if (facet_positive(m, cc, 0, l[0], e[0], x, y, z, retests)) next = __float_as_int(R.nb.x);
-                else if (facet_positive(m, cc, 1, l[1], e[1], x, y, z, retests)) next = __float_as_int(R.nb.y);
-                else if (facet_positive(m, cc, 2, l[2], e[2], x, y, z, retests)) next = __float_as_int(R.nb.z);
-                else if (facet_positive(m, cc, 3, l[3], e[3], x, y, z, retests)) next = __float_as_int(R.nb.w);
-                else { end = cc; break; }
-                if (next < 0) { end = next; break; }
-                cc = next;
-            }
+            // with the first cell's record already loaded; the last cell's
+            // lambdas are the deposit's
+            const int end = walk_screened<PERIODIC || !MOVE>(m, x, y, z, c, max_steps, retests, R, have_rec, l);
             if (end == kWalkFail) {
                 raise_device_error(st, PG_ERR_WALK_LIMIT, i);
                 continue;
@@ -235,18 +213,42 @@ __global__ void k_fixed_to_rho(const unsigned long long *__restrict__ fixed, con
     rho[i] = a * dv_inv[i];
 }
 
-// The mixed form's cell records: FP32 barycentric rows 0-2 and the
-// neighbour ids (int bits in the fourth float4).
-__global__ void k_float_tables(const double *__restrict__ bary, const int4 *__restrict__ nbr, int32_t nc,
-                               float4 *__restrict__ cell_f) {
+// Cell records (FP32 barycentric rows 0-2 and the neighbour ids as int bits)
+// and, in *lam_abs, the largest absolute distance over all cells and facets
+// between lambda_f as the FP64 rows give it and the facet's plane value over
+// its height, at points with coordinates up to X: the rounding of the two
+// FP64 tables (a row's constant term comes from cancelling products, so its
+// error does not shrink with the terms that remain at a point) and of an FP64
+// plane evaluation.
+__global__ void k_float_tables(const double *__restrict__ bary, const double *__restrict__ planes,
+                               const int4 *__restrict__ nbr, int32_t nc, double X, float4 *__restrict__ cell_f,
+                               unsigned *__restrict__ lam_abs) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nc) return;
-    const double *A = bary + 12 * (size_t)c;
-    for (int k = 0; k < 3; ++k)
-        cell_f[4 * (size_t)c + k] = make_float4((float)A[4 * k], (float)A[4 * k + 1], (float)A[4 * k + 2], (float)A[4 * k + 3]);
-    const int4 nb = nbr[c];
-    cell_f[4 * (size_t)c + 3] = make_float4(__int_as_float(nb.x), __int_as_float(nb.y), __int_as_float(nb.z),
-                                            __int_as_float(nb.w));
+    float worst = 0.0f;
+    if (c < nc) {
+        const double *A = bary + 12 * (size_t)c;
+        for (int k = 0; k < 3; ++k)
+            cell_f[4 * (size_t)c + k] = make_float4((float)A[4 * k], (float)A[4 * k + 1], (float)A[4 * k + 2], (float)A[4 * k + 3]);
+        const int4 nb = nbr[c];
+        cell_f[4 * (size_t)c + 3] = make_float4(__int_as_float(nb.x), __int_as_float(nb.y), __int_as_float(nb.z),
+                                                __int_as_float(nb.w));
+        for (int f = 0; f < 4; ++f) {
+            double r[4];
+            for (int j = 0; j < 4; ++j)
+                r[j] = f < 3 ? A[4 * f + j] : (j == 0 ? 1.0 : 0.0) - A[j] - A[4 + j] - A[8 + j];
+            const double *P = planes + 16 * (size_t)c + 4 * f;
+            // lambda_f = -plane_f / height: the height from the gradients
+            const double s = -(r[1] * P[1] + r[2] * P[2] + r[3] * P[3]) / (P[1] * P[1] + P[2] * P[2] + P[3] * P[3]);
+            double d = fabs(r[0] + s * P[0]), t = fabs(r[0]);
+            for (int j = 1; j < 4; ++j) {
+                d += fabs(r[j] + s * P[j]) * X;
+                t += fabs(r[j]) * X;
+            }
+            worst = fmaxf(worst, (float)(2.0 * d + 16.0 * 0x1p-53 * t));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+    if ((threadIdx.x & 31) == 0 && worst > 0.0f) atomicMax(lam_abs, __float_as_uint(worst));
 }
 
 inline int grid_for(int64_t n, int max_blocks) {
@@ -304,9 +306,12 @@ void launch_fixed_to_rho(const unsigned long long *fixed, const double *dv_inv, 
     k_fixed_to_rho<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(fixed, dv_inv, unit, n, rho_acc, rho);
 }
 
-void launch_float_tables(const double *bary, const int4 *nbr, int32_t nc, float4 *cell_f, cudaStream_t st) {
+void launch_float_tables(const double *bary, const double *planes, const int4 *nbr, int32_t nc, double X,
+                         float4 *cell_f, float *lam_abs, cudaStream_t st) {
     count_launches(1);
-    k_float_tables<<<(nc + kThreads - 1) / kThreads, kThreads, 0, st>>>(bary, nbr, nc, cell_f);
+    cudaMemsetAsync(lam_abs, 0, sizeof(float), st);
+    k_float_tables<<<(nc + kThreads - 1) / kThreads, kThreads, 0, st>>>(bary, planes, nbr, nc, X, cell_f,
+                                                                       reinterpret_cast<unsigned *>(lam_abs));
 }
 
 }  // namespace pg

@@ -87,17 +87,13 @@ __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, in
                     // accel (punc/include/punc/pusher.h:66-130): Ei *= dt*(q/m);
                     // KE += 0.5*m*v*(v+Ei); v += Ei.
                     const double ax = ex * coef, ay = ey * coef, az = ez * coef;
-                    ke += hm * vx * (vx + ax);
-                    ke += hm * vy * (vy + ay);
-                    ke += hm * vz * (vz + az);
+                    ke = fma(hm, fma(vx, vx + ax, fma(vy, vy + ay, vz * (vz + az))), ke);
                     vx = vx + ax; vy = vy + ay; vz = vz + az;
                 } else {
                     // boris (punc/include/punc/pusher.h:397-510).
                     const double hx = coef * ex, hy = coef * ey, hz = coef * ez;
                     const double mx = vx + hx, my = vy + hy, mz = vz + hz;
-                    ke += hm * mx * mx;
-                    ke += hm * my * my;
-                    ke += hm * mz * mz;
+                    ke = fma(hm, fma(mx, mx, fma(my, my, mz * mz)), ke);
                     double px = mx, py = my, pz = mz;
                     if (HAS_B) {
                         const double t0 = pp.t[s][0], t1 = pp.t[s][1], t2 = pp.t[s][2];
@@ -119,16 +115,16 @@ __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, in
                 // move / move_periodic (punc/include/punc/pusher.h:648-681).
                 x = x + mp.dt * vx; y = y + mp.dt * vy; z = z + mp.dt * vz;
                 if (PERIODIC) {
-                    x = x - mp.Ld[0] * floor(x / mp.Ld[0]);
-                    y = y - mp.Ld[1] * floor(y / mp.Ld[1]);
-                    z = z - mp.Ld[2] * floor(z / mp.Ld[2]);
+                    x = wrap_periodic(x, mp.Ld[0]);
+                    y = wrap_periodic(y, mp.Ld[1]);
+                    z = wrap_periodic(z, mp.Ld[2]);
                 }
                 p.x[i] = x; p.y[i] = y; p.z[i] = z;
             }
         }
         if (WALK) {
             // Population::update (punc/include/punc/population.h:641-699).
-            const int nc = walk_fp64(m, x, y, z, c, max_steps);
+            const int nc = walk_fp64<PERIODIC || !MOVE>(m, x, y, z, c, max_steps);
             if (nc == kWalkFail) {
                 raise_device_error(st, PG_ERR_WALK_LIMIT, i);
                 continue;

@@ -28,6 +28,9 @@ constexpr int kFixedBits = 30;
 constexpr int64_t kMaxMixedSlots = int64_t(1) << (62 - kFixedBits);
 constexpr int kDead = -1;                 // cell id of a free particle slot
 constexpr int kWalkFail = -2147483647;    // walk step limit reached
+// step limit from which a walk may start again near its point (DevMesh::box):
+// a walk crosses a box of 2^31 cells in fewer steps
+constexpr int kBoxWalkLimit = 65536;
 
 struct DevMesh {
     int32_t nc = 0, ndof = 0;
@@ -37,11 +40,14 @@ struct DevMesh {
     const int4 *dofs = nullptr;       // [nc]
     double *E = nullptr;              // [nc][4]
     const double *dv_inv = nullptr;   // [ndof]
-    // mixed form: one 64-byte record per cell, {barycentric rows 0-2 in FP32
-    // (float4 each), neighbours (int4 bits)}: what the walk, the deposit and
-    // the field read, in one aligned pair of sectors; and the FP32 field
+    // one 64-byte record per cell, {barycentric rows 0-2 in FP32 (float4
+    // each), neighbours (int4 bits)}: what the walks of both forms and the
+    // mixed form's deposit and field read, in one aligned pair of sectors
     const float4 *cell_f = nullptr;   // [nc][4]
-    float *E_f = nullptr;             // [nc][4]
+    float *E_f = nullptr;             // [nc][4] FP32 field (mixed form)
+    // bound on the rounding of the FP64 tables in lambda (launch_float_tables),
+    // for points within lam_range of the origin in every coordinate
+    float lam_abs = 0.0f;
     // CG1 (vertex) field of the ESolver path: [ndof][4] (x, y, z, 0)
     const double *Ev = nullptr;
     const float *Evf = nullptr;
@@ -53,6 +59,10 @@ struct DevMesh {
     // point location considers cells in [loc_lo, loc_hi) only (batched runs
     // whose meshes overlap in space)
     int32_t loc_lo = 0, loc_hi = 0x7fffffff;
+    // 1: the cells fill the bounding box, so a walk may start again near its
+    // point (walk_screened); FP32 copies of the bins' origin and 1 / width
+    int32_t box = 0;
+    float lo_f[3] = {0, 0, 0}, bin_inv_f[3] = {1, 1, 1};
 };
 
 struct DevParticles {
@@ -409,7 +419,8 @@ void launch_kinetic_mixed(const DevParticles &p, int64_t n_slots, const MixedPar
                           int nblocks, double *ke_out, cudaStream_t st);
 void launch_fixed_to_rho(const unsigned long long *fixed, const double *dv_inv, double unit, int32_t n,
                          double *rho_acc, double *rho, cudaStream_t st);
-void launch_float_tables(const double *bary, const int4 *nbr, int32_t nc, float4 *cell_f, cudaStream_t st);
+void launch_float_tables(const double *bary, const double *planes, const int4 *nbr, int32_t nc, double X,
+                         float4 *cell_f, float *lam_abs, cudaStream_t st);
 void launch_image_charge(const DevMesh &m, const double *phi, const double *ofacets, int32_t n_ofacets,
                          int32_t n_obj, double eps0, double *out, cudaStream_t st);
 

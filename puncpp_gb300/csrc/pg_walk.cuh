@@ -21,57 +21,48 @@ __device__ __forceinline__ double plane64(double c0, double c1, double c2, doubl
     return __dadd_rn(d, __dmul_rn(c3, z));
 }
 
-// relocate_fast (punc/include/punc/population.h:539-569) as a bounded loop:
-// the first facet i (0..3) with a positive plane value moves the walk to
-// neighbour i or ends it with -tag; no positive facet ends it in the cell.
-__device__ __forceinline__ int walk_fp64(const DevMesh &m, double x, double y, double z, int c, int max_steps) {
-    for (int it = 0; it < max_steps; ++it) {
-        const double2 *P = reinterpret_cast<const double2 *>(m.planes) + 8 * (size_t)c;
-        const double2 q0 = __ldg(P + 0), q1 = __ldg(P + 1), q2 = __ldg(P + 2), q3 = __ldg(P + 3);
-        const double2 q4 = __ldg(P + 4), q5 = __ldg(P + 5), q6 = __ldg(P + 6), q7 = __ldg(P + 7);
-        const int4 nb = __ldg(m.nbr + c);
-        const double d0 = plane64(q0.x, q0.y, q1.x, q1.y, x, y, z);
-        const double d1 = plane64(q2.x, q2.y, q3.x, q3.y, x, y, z);
-        const double d2 = plane64(q4.x, q4.y, q5.x, q5.y, x, y, z);
-        const double d3 = plane64(q6.x, q6.y, q7.x, q7.y, x, y, z);
-        int next;
-        if (d0 > 0) next = nb.x;
-        else if (d1 > 0) next = nb.y;
-        else if (d2 > 0) next = nb.z;
-        else if (d3 > 0) next = nb.w;
-        else return c;
-        if (next < 0) return next;
-        c = next;
-    }
-    return kWalkFail;
-}
-
+// relocate_fast (punc/include/punc/population.h:539-569) as a bounded loop
+// (walk_fp64, walk_mixed below): the first facet i (0..3) with a positive
+// plane value moves the walk to neighbour i or ends it with -tag; no positive
+// facet ends it in the cell.
 // Relative bound on |FP32 affine value - exact value| in units of the sum of
-// the terms' magnitudes: one rounding per coefficient and per fmaf, with a
-// factor two of slack.
+// the terms' magnitudes: one rounding per coefficient, coordinate and fmaf
+// (at most five), and slack.  The absolute part of the bound is the mesh's
+// (DevMesh::lam_abs, the rounding of the FP64 tables).
 constexpr float kPlaneEps = 8.0f * 5.9604645e-08f;   // 8 * 2^-24
 
+// Cell record of c: barycentric rows 0-2 in FP32 and the neighbours (int bits).
+struct CellRec {
+    float4 r0, r1, r2, nb;
+};
+__device__ __forceinline__ CellRec load_rec(const DevMesh &m, int c) {
+    const float4 *R = m.cell_f + 4 * (size_t)c;
+    return CellRec{__ldg(R), __ldg(R + 1), __ldg(R + 2), __ldg(R + 3)};
+}
+
 // Barycentric coordinates of the FP32 point from a cell record's rows 0-2
-// (the fourth is 1 - l0 - l1 - l2) and bounds on their FP32 errors.
-__device__ __forceinline__ void lambdas_f32(const float4 r0, const float4 r1, const float4 r2, float x, float y,
-                                            float z, float l[4], float e[4]) {
-    const float4 r[3] = {r0, r1, r2};
+// (the fourth is 1 - l0 - l1 - l2) and bounds on their distance from the
+// FP64 planes' values over the heights, at the FP32 point and at any FP64
+// point that rounds to it.
+__device__ __forceinline__ void lambdas_f32(const DevMesh &m, const CellRec &R, float x, float y, float z, float l[4],
+                                            float e[4]) {
+    const float4 r[3] = {R.r0, R.r1, R.r2};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         l[k] = fmaf(r[k].w, z, fmaf(r[k].z, y, fmaf(r[k].y, x, r[k].x)));
-        e[k] = kPlaneEps * (fabsf(r[k].x) + fabsf(r[k].y * x) + fabsf(r[k].z * y) + fabsf(r[k].w * z));
+        e[k] = fmaf(kPlaneEps, fabsf(r[k].x) + fabsf(r[k].y * x) + fabsf(r[k].z * y) + fabsf(r[k].w * z), m.lam_abs);
     }
     l[3] = __fsub_rn(__fsub_rn(__fsub_rn(1.0f, l[0]), l[1]), l[2]);
     e[3] = e[0] + e[1] + e[2] + kPlaneEps * (1.0f + fabsf(l[0]) + fabsf(l[1]) + fabsf(l[2]));
 }
 
-// Is the FP32 point outside facet f (opposite local vertex f, where lambda_f
-// = 0)?  Decided from the sign of lambda_f when it exceeds its error bound
-// (lambda_f < 0 exactly when the facet's plane value is positive); otherwise
-// re-tested in FP64 with the FP64 plane, the exact FP64 predicate at this
-// point.
-__device__ __forceinline__ bool facet_positive(const DevMesh &m, int c, int f, float l, float e, float x, float y,
-                                               float z, int &retests) {
+// Is the point outside facet f (opposite local vertex f, where lambda_f = 0)?
+// Decided from the sign of lambda_f when it exceeds its error bound (lambda_f
+// < 0 exactly when the facet's plane value is positive); otherwise re-tested
+// in FP64 with the FP64 plane, the exact FP64 predicate at this point.
+template <class T>
+__device__ __forceinline__ bool facet_positive(const DevMesh &m, int c, int f, float l, float e, T x, T y, T z,
+                                               int &retests) {
     if (l < -e) return true;
     if (l > e) return false;
     ++retests;
@@ -80,26 +71,114 @@ __device__ __forceinline__ bool facet_positive(const DevMesh &m, int c, int f, f
     return plane64(a.x, a.y, b.x, b.y, (double)x, (double)y, (double)z) > 0;
 }
 
-// The walk of the mixed form: same facet order and semantics as walk_fp64,
-// every decision equal to the FP64 predicate at the FP32 position.  Reads
-// one 64-byte cell record per cell visited.
-__device__ __forceinline__ int walk_mixed(const DevMesh &m, float x, float y, float z, int c, int max_steps,
-                                          int &retests) {
+// A cell near the point: the last cell of the point's location bin.
+__device__ __forceinline__ int near_cell(const DevMesh &m, float x, float y, float z) {
+    const float u[3] = {x, y, z};
+    int b[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int k = (int)((u[j] - m.lo_f[j]) * m.bin_inv_f[j]);
+        b[j] = k < 0 ? 0 : (k >= m.nbin[j] ? m.nbin[j] - 1 : k);
+    }
+    const int64_t bin = ((int64_t)b[0] * m.nbin[1] + b[1]) * m.nbin[2] + b[2];
+    return __ldg(m.bin_cells + __ldg(m.bin_ptr + bin + 1) - 1);
+}
+
+// The point lies this many facet heights or more beyond some facet of the
+// first cell: a walk of about as many cells.  Periodic moves wrap a particle
+// to the other side of the box, which is a walk through every cell between,
+// and its warp waits for it (24^3 cells, 663k thermal electrons: the FP64 pass
+// 2.44 ms with long FP64 walks, 0.24 ms now).
+constexpr float kFarLambda = -6.0f;
+constexpr int kNearSteps = 256;
+
+// The walk of relocate_fast (walk_fp64) with each facet decided in FP32 where
+// its error bound allows, every decision equal to the FP64 predicate at the
+// point (T: double or float).  One 64-byte record per cell visited instead of
+// 144 bytes, and no FP64 operation outside the bound (a plane test is six, at
+// 1/64 of the FP32 rate; the FP64 pass over 1.5M particles at 53^3 cells 525
+// us with them, 224 without).  R, have_rec: the first cell's record when the
+// caller has it; R and l are the last cell's on return.
+//
+// NEAR: in a mesh whose cells fill their bounding box (m.box; set only with a
+// step limit that no walk through such a mesh reaches) a walk that starts far
+// from its point starts again at a cell near it.  The result counts only if the
+// point lies inside its cell by more than the error bounds: that cell is then
+// the only one whose four plane values are not positive, the one where the
+// long walk ends too.  Otherwise the long walk runs.
+template <bool NEAR, class T>
+__device__ __forceinline__ int walk_screened(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
+                                             CellRec &R, bool have_rec, float l[4]) {
+    const float xf = (float)x, yf = (float)y, zf = (float)z;
+    int cc = c;
+    bool near_walk = false, may_restart = NEAR && m.box != 0;
     for (int it = 0; it < max_steps; ++it) {
-        const float4 *R = m.cell_f + 4 * (size_t)c;
-        const float4 r0 = __ldg(R), r1 = __ldg(R + 1), r2 = __ldg(R + 2), rn = __ldg(R + 3);
-        float l[4], e[4];
-        lambdas_f32(r0, r1, r2, x, y, z, l, e);
+        float e[4];
+        if (!have_rec) R = load_rec(m, cc);
+        have_rec = false;
+        lambdas_f32(m, R, xf, yf, zf, l, e);
+        if (NEAR && may_restart && fminf(fminf(l[0], l[1]), fminf(l[2], l[3])) < kFarLambda) {
+            cc = near_cell(m, xf, yf, zf);
+            near_walk = true;
+            may_restart = false;
+            continue;
+        }
+        may_restart = false;
         int next;
-        if (facet_positive(m, c, 0, l[0], e[0], x, y, z, retests)) next = __float_as_int(rn.x);
-        else if (facet_positive(m, c, 1, l[1], e[1], x, y, z, retests)) next = __float_as_int(rn.y);
-        else if (facet_positive(m, c, 2, l[2], e[2], x, y, z, retests)) next = __float_as_int(rn.z);
-        else if (facet_positive(m, c, 3, l[3], e[3], x, y, z, retests)) next = __float_as_int(rn.w);
-        else return c;
-        if (next < 0) return next;
-        c = next;
+        bool stay = false;
+        if (facet_positive(m, cc, 0, l[0], e[0], x, y, z, retests)) next = __float_as_int(R.nb.x);
+        else if (facet_positive(m, cc, 1, l[1], e[1], x, y, z, retests)) next = __float_as_int(R.nb.y);
+        else if (facet_positive(m, cc, 2, l[2], e[2], x, y, z, retests)) next = __float_as_int(R.nb.z);
+        else if (facet_positive(m, cc, 3, l[3], e[3], x, y, z, retests)) next = __float_as_int(R.nb.w);
+        else { next = cc; stay = true; }
+        if (NEAR && near_walk) {
+            const bool sure = stay && l[0] > e[0] && l[1] > e[1] && l[2] > e[2] && l[3] > e[3];
+            if (sure) return cc;
+            if (stay || next < 0 || it >= kNearSteps) {
+                near_walk = false;
+                cc = c;
+                it = -1;
+                continue;
+            }
+        } else {
+            if (stay) return cc;
+            if (next < 0) return next;
+        }
+        cc = next;
     }
     return kWalkFail;
+}
+
+__device__ __forceinline__ int walk_mixed(const DevMesh &m, float x, float y, float z, int c, int max_steps,
+                                          int &retests) {
+    CellRec R;
+    float l[4];
+    return walk_screened<false>(m, x, y, z, c, max_steps, retests, R, false, l);
+}
+
+template <bool NEAR>
+__device__ __forceinline__ int walk_fp64(const DevMesh &m, double x, double y, double z, int c, int max_steps) {
+    CellRec R;
+    float l[4];
+    int retests = 0;
+    return walk_screened<NEAR>(m, x, y, z, c, max_steps, retests, R, false, l);
+}
+
+// x - L floor(x / L), one coordinate of move_periodic
+// (punc/include/punc/pusher.h:666-681), without the division where the
+// quotient's floor is known to be 0, 1 or -1: for 0 < x < L, L <= x < 2 L and
+// -L <= x <= -1e-200 the rounded quotient stays on its side of the integers
+// (it has a neighbour of the integer between), so the results are the same
+// bits.  The first test, the common one, is an integer comparison (positive
+// doubles order as their bits).  L must lie in (0, 1e100].
+__device__ __forceinline__ double wrap_periodic(double x, double L) {
+    const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
+    if (bx - 1 < (unsigned long long)__double_as_longlong(L) - 1) return x;
+    if (L > 0.0 && L <= 1e100) {
+        if (x >= L && x < 2.0 * L) return __dadd_rn(x, -L);
+        if (x <= -1e-200 && x >= -L) return __dadd_rn(x, L);
+    }
+    return __dadd_rn(x, -__dmul_rn(L, floor(__ddiv_rn(x, L))));
 }
 
 // __float2ll_rn(v) for finite |v| < 2^62 on the 32-bit conversion path:
