@@ -416,149 +416,180 @@ std::vector<std::vector<int>> charge_sharing_sets(std::vector<pg_source> vs, int
 
 // ---- solver internals ------------------------------------------------------
 
-// Lanes per row of an AMG operator: SELL-32 with one thread per row up to 12
-// entries a row on average, else CSR with a power of two of lanes (at most
-// 512, the block) giving each lane three to six entries.
-// Lanes per row for an operator applied by `threads` threads of the
-// cooperative PCG: the choice with the shortest chain of dependent memory
-// round trips per thread, the quantity that bounds a latency-bound phase.
-// g == 1: SELL-32, one thread per row, four rows and two entries of each per
-// step; g = 2..32: CSR, g lanes per row, four rows per lane group, two entries
-// per lane per step; g = 64..512: the warps of one block per row, four
-// entries per lane per step.  A round (rows of one pass) costs one trip for
-// the row offsets plus two (column, then value gathered) per step.
-static int lanes_per_row(const Csr &A, int64_t threads) {
-    const double n = (double)std::max<int64_t>(1, A.n);
-    double avg = A.n > 0 ? (double)A.ci.size() / n : 0.0, wmax = 0.0;
-    for (int64_t r = 0; r < A.n; ++r) wmax = std::max(wmax, (double)(A.rp[r + 1] - A.rp[r]));
-    const double T = (double)std::max<int64_t>(threads, 32);
-    auto chain = [&](int g) {
-        if (g == 1) {
-            // SELL slices pad to their longest row
-            const double rounds = std::ceil(n / T / 4.0), steps = std::ceil(std::min(wmax, 1.25 * avg) / 2.0);
-            return rounds * (1.0 + 2.0 * steps);
-        }
-        if (g <= 32) {
-            const double groups = std::floor(T / g), rounds = std::ceil(n / groups / 4.0);
-            return rounds * (1.0 + 2.0 * std::ceil(avg / g / 2.0));
-        }
-        const double per_round = std::floor(T / g), rounds = std::ceil(n / per_round);
-        return rounds * (2.0 + 2.0 * std::ceil(avg / g / 4.0));   // + the block's partial-sum barriers
-    };
-    int best = avg <= 12.0 ? 1 : 2;
-    double bc = chain(best);
-    for (int g = 2; g <= 512; g *= 2) {
-        const double c = chain(g);
-        if (c < bc - 1e-9) { bc = c; best = g; }
-    }
-    return best;
+// Lanes per row of a CSR operator of the device cycle: the smallest power of
+// two, 2 to 512, that leaves each lane at most three chunks of its row on
+// average.  Fewer lanes lengthen a row's chain of loads, more leave lanes idle
+// and cost shuffles.  Measured on the 80^3 probe's solve: S_0^T (18 chunks a
+// row) 1.656 / 1.628 / 1.605 / 1.668 / 1.847 ms with 2 / 4 / 8 / 16 / 32 lanes; U1
+// (7) 1.657 / 1.628 / 1.641 / 1.688 with 2 / 4 / 8 / 16; S_1^T (147) 1.720 / 1.635 /
+// 1.653 / 1.677 / 1.794 with 16 / 32 / 64 / 128 / 256; on the 40^3 one A_1 (8) 0.620 /
+// 0.623 / 0.668 / 0.770 with 2 / 4 / 8 / 16.
+static int lanes_per_row(const Csr &A) {
+    double chunks = 0.0;
+    for (int64_t r = 0; r < A.n; ++r) chunks += (double)((A.rp[r + 1] - A.rp[r] + 3) / 4);
+    chunks /= (double)std::max<int64_t>(1, A.n);
+    int g = 2;
+    while (g < 512 && chunks > 3.0 * g) g *= 2;
+    return g;
 }
 
-// Upload a CSR operator: SELL-32 (padding: the slice's first column, value
-// 0) when g == 1, else CSR.  c16: 16-bit column offsets from the smallest
-// column of each slice (SELL) or row (CSR), when every span fits in 16 bits;
-// v16: IEEE binary16 values of v / vscale with vscale = max|v| / 1024 (the
-// preconditioner's operators; binary16 keeps 11 significant bits, and halving
-// the bytes keeps the hierarchy of large meshes resident in L2).
-static int upload_op(pg_sim *s, const Csr &A, int g, SpOp &out, bool want_c16 = false, bool want_v16 = false) {
-    const int64_t n = A.n;
-    int rc;
+// Upload a CSR operator in chunks of four entries (SpOp).  half: binary16
+// values of v / vscale with vscale = max|v| / 1024 (the preconditioner's
+// transfer and coarse operators; binary16 keeps 11 significant bits, and
+// halving the bytes keeps the hierarchy of large meshes resident in L2).
+// Columns are 16-bit offsets from the smallest column of each slice (g == 1)
+// or row when that is wanted and every span fits in 16 bits.
+static int upload_op(pg_sim *s, const Csr &A, int g, SpOp &out, bool half, bool want_c16 = true) {
+    const int64_t n = A.n, rows = g == 1 ? 32 : 1, units = (n + rows - 1) / rows;
+    std::vector<int32_t> head(2 * (size_t)(units + 1), 0);
+    int64_t chunks = 0;
+    bool c16 = want_c16;
+    for (int64_t u = 0; u < units; ++u) {
+        int64_t w = 0;
+        int32_t lo = INT32_MAX, hi = 0;
+        for (int64_t r = rows * u; r < std::min(n, rows * (u + 1)); ++r) {
+            w = std::max(w, (A.rp[r + 1] - A.rp[r] + 3) / 4);
+            for (int64_t k = A.rp[r]; k < A.rp[r + 1]; ++k) { lo = std::min(lo, A.ci[k]); hi = std::max(hi, A.ci[k]); }
+        }
+        if (lo > hi) lo = hi = 0;
+        c16 = c16 && hi - lo <= 65535;
+        head[2 * u] = (int32_t)chunks;
+        head[2 * u + 1] = lo;
+        chunks += rows * w;
+        if (4 * chunks > (int64_t)INT32_MAX) return fail(PG_ERR_ARG, "operator with 2^31 or more stored entries");
+    }
+    head[2 * units] = (int32_t)chunks;
+    const size_t slots = 4 * (size_t)std::max<int64_t>(1, chunks);
+    double scale = 1.0;
+    if (half) {
+        double vmax = 0.0;
+        for (double v : A.v) vmax = std::max(vmax, std::fabs(v));
+        if (vmax > 0.0) scale = vmax / 1024.0;
+    }
     out = SpOp{};
     out.n = (int32_t)n;
     out.g = g;
-    std::vector<int64_t> ptr;     // slice or row offsets
-    std::vector<int32_t> swidth;
-    std::vector<int32_t> col;
-    std::vector<double> val;
-    std::vector<int32_t> base;    // smallest column per slice or row
-    if (g > 1) {
-        ptr.assign(A.rp.begin(), A.rp.end());
-        col.assign(A.ci.begin(), A.ci.end());
-        val.assign(A.v.begin(), A.v.end());
-        base.assign(n, 0);
-        for (int64_t r = 0; r < n; ++r)
-            if (A.rp[r + 1] > A.rp[r]) base[r] = *std::min_element(A.ci.begin() + A.rp[r], A.ci.begin() + A.rp[r + 1]);
-    } else {
-        const int64_t nsl = (n + 31) / 32;
-        ptr.assign(nsl + 1, 0);
-        swidth.assign(nsl, 0);
-        base.assign(nsl, 0);
-        for (int64_t sl = 0; sl < nsl; ++sl) {
-            int64_t w = 0;
-            int32_t b = INT32_MAX;
-            for (int64_t r = 32 * sl; r < std::min(n, 32 * sl + 32); ++r) {
-                w = std::max(w, A.rp[r + 1] - A.rp[r]);
-                for (int64_t k = A.rp[r]; k < A.rp[r + 1]; ++k) b = std::min(b, A.ci[k]);
+    out.c16 = c16 ? 1 : 0;
+    out.half = half ? 1 : 0;
+    out.vscale = (float)scale;
+    out.chunks = (int32_t)chunks;
+    int rc;
+    int32_t *d_head;
+    if ((rc = upload(s, &d_head, head))) return rc;
+    out.head = reinterpret_cast<const int2 *>(d_head);
+    // f(slot, unit, entry) for every stored entry: SELL rows in order, CSR rows
+    // dealt out over their m chunks (entry j in chunk j % m), so that the lanes
+    // of a row gather consecutive columns together
+    auto each = [&](auto f) {
+        for (int64_t r = 0; r < n; ++r) {
+            const int64_t u = r / rows, lane = r % rows, m = (A.rp[r + 1] - A.rp[r] + 3) / 4;
+            for (int64_t k = A.rp[r]; k < A.rp[r + 1]; ++k) {
+                const int64_t j = k - A.rp[r];
+                const int64_t chunk = g == 1 ? (j / 4) * rows + lane : j % m, e = g == 1 ? j % 4 : j / m;
+                f(4 * ((size_t)head[2 * u] + (size_t)chunk) + e, u, k);
             }
-            swidth[sl] = (int32_t)w;
-            base[sl] = b == INT32_MAX ? 0 : b;
-            ptr[sl + 1] = ptr[sl] + 32 * w;
         }
-        col.assign(std::max<int64_t>(1, ptr[nsl]), 0);
-        val.assign(std::max<int64_t>(1, ptr[nsl]), 0.0);
-        for (int64_t sl = 0; sl < nsl; ++sl)
-            for (int64_t o = ptr[sl]; o < ptr[sl + 1]; ++o) col[o] = base[sl];
-        for (int64_t sl = 0; sl < nsl; ++sl)
-            for (int lane = 0; lane < 32; ++lane) {
-                const int64_t r = 32 * sl + lane;
-                if (r >= n) continue;
-                const int64_t len = A.rp[r + 1] - A.rp[r];
-                for (int64_t k = 0; k < len; ++k) {
-                    const int64_t o = ptr[sl] + 32 * k + lane;
-                    col[o] = A.ci[A.rp[r] + k];
-                    val[o] = A.v[A.rp[r] + k];
-                }
+    };
+    auto half_of = [&](int64_t k) { return (uint32_t)__half_as_ushort(__float2half_rn((float)(A.v[k] / scale))); };
+    auto put = [&](auto &host, const void *&dst) -> int {
+        typename std::decay<decltype(host)>::type::value_type *d = nullptr;
+        const int e = upload(s, &d, host);
+        dst = d;
+        return e;
+    };
+    if (half && c16) {
+        std::vector<uint32_t> pk(slots, 0u);
+        each([&](size_t o, int64_t u, int64_t k) { pk[o] = (half_of(k) << 16) | (uint32_t)(A.ci[k] - head[2 * u + 1]); });
+        return put(pk, out.val);
+    }
+    if (half) {
+        std::vector<uint16_t> v(slots, 0);
+        each([&](size_t o, int64_t, int64_t k) { v[o] = (uint16_t)half_of(k); });
+        if ((rc = put(v, out.val))) return rc;
+    } else {
+        std::vector<float> v(slots, 0.0f);
+        each([&](size_t o, int64_t, int64_t k) { v[o] = (float)A.v[k]; });
+        if ((rc = put(v, out.val))) return rc;
+    }
+    if (c16) {
+        std::vector<uint16_t> c(slots, 0);
+        each([&](size_t o, int64_t u, int64_t k) { c[o] = (uint16_t)(A.ci[k] - head[2 * u + 1]); });
+        return put(c, out.col);
+    }
+    // 32-bit columns: padding points at a column of its unit
+    std::vector<int32_t> c(slots, 0);
+    for (int64_t u = 0; u < units; ++u)
+        for (size_t o = 4 * (size_t)head[2 * u]; o < 4 * (size_t)head[2 * u + 2]; ++o) c[o] = head[2 * u + 1];
+    each([&](size_t o, int64_t, int64_t k) { c[o] = A.ci[k]; });
+    return put(c, out.col);
+}
+
+// The solver's FP32 matrix for the device cycle: SELL-32 of its off-diagonal
+// entries in pairs (val: two values, col: two columns; heads as SpOp's, in
+// pairs) and its diagonal.
+static int upload_a0(pg_sim *s, const Csr &A, SpOp &out, const float **diag) {
+    const int64_t n = A.n, units = (n + 31) / 32;
+    std::vector<int32_t> head(2 * (size_t)(units + 1), 0);
+    std::vector<float> d(std::max<int64_t>(1, n), 0.0f);
+    int64_t pairs = 0;
+    bool c16 = true;
+    for (int64_t u = 0; u < units; ++u) {
+        int64_t w = 0;
+        int32_t lo = INT32_MAX, hi = 0;
+        for (int64_t r = 32 * u; r < std::min(n, 32 * (u + 1)); ++r) {
+            int64_t len = 0;
+            for (int64_t k = A.rp[r]; k < A.rp[r + 1]; ++k) {
+                if (A.ci[k] == r) { d[r] = (float)A.v[k]; continue; }
+                ++len;
+                lo = std::min(lo, A.ci[k]);
+                hi = std::max(hi, A.ci[k]);
             }
+            w = std::max(w, (len + 1) / 2);
+        }
+        if (lo > hi) lo = hi = 0;
+        c16 = c16 && hi - lo <= 65535;
+        head[2 * u] = (int32_t)pairs;
+        head[2 * u + 1] = lo;
+        pairs += 32 * w;
+        if (2 * pairs > (int64_t)INT32_MAX) return fail(PG_ERR_ARG, "operator with 2^31 or more stored entries");
     }
-    if (ptr.back() > (int64_t)INT32_MAX) return fail(PG_ERR_ARG, "operator with 2^31 or more stored entries");
-    if (col.empty()) col.push_back(0);
-    if (val.empty()) val.push_back(0.0);
-    bool c16 = want_c16;
+    head[2 * units] = (int32_t)pairs;
+    const size_t slots = 2 * (size_t)std::max<int64_t>(1, pairs);
+    std::vector<float> v(slots, 0.0f);
+    std::vector<int32_t> c(slots, 0);   // offsets (16-bit form) or columns; padding: the slice's smallest
+    for (int64_t u = 0; u < units; ++u) {
+        const int32_t base = c16 ? 0 : head[2 * u + 1], sub = c16 ? head[2 * u + 1] : 0;
+        for (size_t o = 2 * (size_t)head[2 * u]; o < 2 * (size_t)head[2 * u + 2]; ++o) c[o] = base;
+        for (int64_t r = 32 * u; r < std::min(n, 32 * (u + 1)); ++r) {
+            int64_t j = 0;
+            for (int64_t k = A.rp[r]; k < A.rp[r + 1]; ++k) {
+                if (A.ci[k] == r) continue;
+                const size_t o = 2 * ((size_t)head[2 * u] + (size_t)(j / 2) * 32 + (r & 31)) + (j & 1);
+                v[o] = (float)A.v[k];
+                c[o] = A.ci[k] - sub;
+                ++j;
+            }
+        }
+    }
+    out = SpOp{};
+    out.n = (int32_t)n;
+    out.c16 = c16 ? 1 : 0;
+    int rc;
+    int32_t *d_head;
+    float *d_v, *d_d;
+    if ((rc = upload(s, &d_head, head)) || (rc = upload(s, &d_v, v)) || (rc = upload(s, &d_d, d))) return rc;
+    out.head = reinterpret_cast<const int2 *>(d_head);
+    out.val = d_v;
+    *diag = d_d;
     if (c16) {
-        const int64_t units = (int64_t)base.size();
-        for (int64_t u = 0; u < units && c16; ++u)
-            for (int64_t o = ptr[u]; o < ptr[u + 1]; ++o)
-                if ((int64_t)col[o] - base[u] > 65535) { c16 = false; break; }
-    }
-    int64_t *d_ptr;
-    if ((rc = upload(s, &d_ptr, ptr))) return rc;
-    out.ptr = d_ptr;
-    if (g == 1) {
-        int32_t *d_sw;
-        if ((rc = upload(s, &d_sw, swidth))) return rc;
-        out.swidth = d_sw;
-        out.wmax = swidth.empty() ? 0 : *std::max_element(swidth.begin(), swidth.end());
-    }
-    if (c16) {
-        std::vector<uint16_t> c(col.size(), 0);
-        const int64_t units = (int64_t)base.size();
-        for (int64_t u = 0; u < units; ++u)
-            for (int64_t o = ptr[u]; o < ptr[u + 1]; ++o) c[o] = (uint16_t)(col[o] - base[u]);
+        std::vector<uint16_t> c2(c.begin(), c.end());
         uint16_t *d_c;
-        int32_t *d_b;
-        if ((rc = upload(s, &d_c, c)) || (rc = upload(s, &d_b, base))) return rc;
-        out.col16 = d_c;
-        out.cbase = d_b;
+        if ((rc = upload(s, &d_c, c2))) return rc;
+        out.col = d_c;
     } else {
-        int32_t *d_col;
-        if ((rc = upload(s, &d_col, col))) return rc;
-        out.col = d_col;
-    }
-    if (want_v16) {
-        double vmax = 0.0;
-        for (double v : val) vmax = std::max(vmax, std::fabs(v));
-        const double sc = vmax > 0.0 ? vmax / 1024.0 : 1.0;
-        std::vector<uint16_t> h(val.size());
-        for (size_t k = 0; k < val.size(); ++k) h[k] = __half_as_ushort(__float2half_rn((float)(val[k] / sc)));
-        uint16_t *d_h;
-        if ((rc = upload(s, &d_h, h))) return rc;
-        out.val16 = d_h;
-        out.vscale = (float)sc;
-    } else {
-        std::vector<float> v32(val.begin(), val.end());
-        float *d_val;
-        if ((rc = upload(s, &d_val, v32))) return rc;
-        out.val = d_val;
+        int32_t *d_c;
+        if ((rc = upload(s, &d_c, c))) return rc;
+        out.col = d_c;
     }
     return PG_OK;
 }
@@ -582,9 +613,6 @@ static int build_amg(pg_sim *s) {
     s->amg_nnz_u1 = (int64_t)cyc.U1.ci.size();
     AmgDev &M = s->amg;
     M = AmgDev{};
-    // threads of the solve's grid (fewer blocks for small systems)
-    const int64_t gt = (int64_t)std::min<int64_t>(pcg_amg_grid_blocks(), (A0.n + kPcgThreads - 1) / kPcgThreads) *
-                       kPcgThreads;
     M.nlev = (int32_t)h.levels.size();
     const int L = M.nlev - 1;
     s->amg_rows.assign(M.nlev, 0);
@@ -592,7 +620,7 @@ static int build_amg(pg_sim *s) {
     s->amg_nnz_p.assign(M.nlev, 0);
     int rc;
     if (L >= 1 && (rc = dalloc(s, &M.stack, cyc.stack_len))) return rc;
-    if ((rc = dalloc(s, &M.r_alt, h.levels[0].A.n))) return rc;
+    if ((rc = dalloc(s, &M.s0, h.levels[0].A.n))) return rc;
     for (int l = 0; l < M.nlev; ++l) {
         const AmgLevel &Lv = h.levels[l];
         s->amg_rows[l] = Lv.A.n;
@@ -602,21 +630,22 @@ static int build_amg(pg_sim *s) {
         if (l == 0) {
             // the PCG's own product A p reads level 0's operator, also when
             // L == 0: FP32 values (the Krylov recurrence), 16-bit columns
-            if ((rc = upload_op(s, Lv.A, 1, D.A, true, false))) return rc;
+            if ((rc = upload_a0(s, Lv.A, D.A, &M.diag0))) return rc;
             D.dinv = s->A_dinv32;
         }
         if (l == L) break;   // the coarsest level lives in G (or cinv when L == 0)
         if (l > 0) {
-            if ((rc = upload_op(s, Lv.A, lanes_per_row(Lv.A, gt), D.A, true, true))) return rc;
+            if ((rc = upload_op(s, Lv.A, lanes_per_row(Lv.A), D.A, true))) return rc;
             std::vector<float> dinv(Lv.dinv.begin(), Lv.dinv.end());
             float *d_dinv;
-            if ((rc = upload(s, &d_dinv, dinv)) || (rc = dalloc(s, &D.b, Lv.A.n))) return rc;
+            if ((rc = upload(s, &d_dinv, dinv)) || (rc = dalloc(s, &D.b, Lv.A.n)) || (rc = dalloc(s, &D.sb, Lv.A.n)))
+                return rc;
             D.dinv = d_dinv;
         }
         D.omega = (float)Lv.omega;
-        if (l < L - 1 && (rc = upload_op(s, Lv.ST, lanes_per_row(Lv.ST, gt), D.ST, true, true))) return rc;
+        if (l < L - 1 && (rc = upload_op(s, Lv.ST, lanes_per_row(Lv.ST), D.ST, true))) return rc;
         if (l >= 2) D.t = M.stack + cyc.stack_off[l];
-        else if ((rc = dalloc(s, &D.t, Lv.A.n))) return rc;
+        else if (l == 1 && (rc = dalloc(s, &D.t, Lv.A.n))) return rc;
     }
     if (L == 0) {
         // the whole operator is the coarsest: z = C^-1 r
@@ -628,30 +657,31 @@ static int build_amg(pg_sim *s) {
         for (int64_t i = 0; i <= nc; ++i) C.rp[i] = i * nc;
         for (int64_t k = 0; k < nc * nc; ++k) C.ci[k] = (int32_t)(k % nc);
         C.v = h.coarse_inv;
-        if ((rc = upload_op(s, C, lanes_per_row(C, gt), M.cinv))) return rc;
+        if ((rc = upload_op(s, C, lanes_per_row(C), M.cinv, false, false))) return rc;
     } else {
-        if ((rc = upload_op(s, h.levels[0].S, lanes_per_row(h.levels[0].S, gt), M.S0, true, true)) ||
-            (rc = upload_op(s, cyc.G, lanes_per_row(cyc.G, gt), M.G)))
+        if ((rc = upload_op(s, h.levels[0].S, 1, M.S0, true)) ||
+            (rc = upload_op(s, cyc.G, lanes_per_row(cyc.G), M.G, false, false)))
             return rc;
         M.yL = L >= 2 ? M.stack + cyc.stack_off[L] : M.stack;
-        if (L >= 2 && ((rc = upload_op(s, cyc.U1, lanes_per_row(cyc.U1, gt), M.U1, true, true)) ||
+        if (L >= 2 && ((rc = upload_op(s, cyc.U1, lanes_per_row(cyc.U1), M.U1, true)) ||
                        (rc = dalloc(s, &M.y1, h.levels[1].A.n))))
             return rc;
     }
     // the solver kernel takes each operator's value format from its role:
     // binary16 for the preconditioner's transfer and coarse operators, FP32
     // for A_0, G and the coarsest inverse
-    bool fmt = M.lev[0].A.val16 == nullptr;
-    for (int l = 1; l < L; ++l) fmt = fmt && M.lev[l].A.val16 != nullptr;
-    for (int l = 0; l + 1 < L; ++l) fmt = fmt && M.lev[l].ST.val16 != nullptr;
-    if (L >= 1) fmt = fmt && M.S0.val16 != nullptr && M.G.val16 == nullptr;
-    if (L >= 2) fmt = fmt && M.U1.val16 != nullptr;
-    if (L == 0) fmt = fmt && M.cinv.val16 == nullptr;
+    bool fmt = !M.lev[0].A.half;
+    for (int l = 1; l < L; ++l) fmt = fmt && M.lev[l].A.half;
+    for (int l = 0; l + 1 < L; ++l) fmt = fmt && M.lev[l].ST.half;
+    if (L >= 1) fmt = fmt && M.S0.half && !M.G.half;
+    if (L >= 2) fmt = fmt && M.U1.half;
+    if (L == 0) fmt = fmt && !M.cinv.half;
     if (!fmt) return fail(PG_ERR_ARG, "AMG: operator value formats differ from the solver's");
     // operator bytes of one iteration: A_0 twice (A p and the level-0
-    // smoother), then each operator of the cycle once
+    // smoother; its diagonal counted as entries), then each operator of the
+    // cycle once
     auto opb = [](const SpOp &o, int64_t entries) {
-        return entries * ((o.col16 ? 2 : 4) + (o.val16 ? 2 : 4));
+        return entries * ((o.c16 ? 2 : 4) + (o.half ? 2 : 4));
     };
     int64_t cb = 2 * opb(M.lev[0].A, (int64_t)h.levels[0].A.ci.size());
     if (L == 0) {
@@ -1252,7 +1282,7 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
             (rc = upload(s, &s->M_val, h.M)) || (rc = upload(s, &s->bc_kind, kind)) || (rc = upload(s, &s->bc_value, gval)) ||
             (rc = upload(s, &s->w_ext, wext)) || (rc = upload(s, &s->w_obj, wobj)))
             return bail(rc);
-        const int nb = std::max(pcg_grid_blocks(), pcg_amg_grid_blocks());
+        const int nb = std::max(pcg_grid_blocks(), 2 * pcg_amg_grid_blocks());
         if ((rc = dalloc(s, &s->r, nd)) || (rc = dalloc(s, &s->z, nd)) || (rc = dalloc(s, &s->p0, nd)) ||
             (rc = dalloc(s, &s->p1, nd)) || (rc = dalloc(s, &s->Ap, nd)) || (rc = dalloc(s, &s->pcg_part, 4 * nb)) ||
             (rc = dalloc(s, &s->pcg_out_i, 2)) || (rc = dalloc(s, &s->pcg_out_d, 2)) ||

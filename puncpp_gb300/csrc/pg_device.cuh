@@ -243,7 +243,7 @@ struct PcgArgs {
     double *p0;
     double *p1;
     double *Ap;
-    double *partials;             // [4][grid]
+    double *partials;             // [6][grid]
     double rtol, atol;
     int32_t max_iter;
     int32_t remove_mean;          // periodic: project b and x onto mean zero
@@ -258,41 +258,44 @@ struct PcgArgs {
     int32_t *out_updates;         // reliable updates done
 };
 
-// AMG hierarchy on the device: FP32 sparse operators, each either SELL-32
-// (one thread per row, g == 1) or CSR processed by g lanes per row (g a power
-// of two: up to 32 within a warp, 64..512 across the warps of one block) for
-// operators with long rows.
+// AMG hierarchy on the device: sparse operators, each either SELL-32 (one
+// thread per row, g == 1) or CSR processed by g lanes per row (g a power of
+// two: up to 32 within a warp, 64..512 across the warps of one block) for
+// operators with long rows.  Entries come in chunks of four (rows padded with
+// zeros), one or two 16-byte loads each: values FP32 or binary16 (times
+// vscale), columns 32-bit or 16-bit offsets from the smallest column of their
+// SELL slice or CSR row.
 struct SpOp {
-    int32_t n = 0;                       // rows
-    int32_t g = 1;                       // lanes per row
-    const int64_t *ptr = nullptr;        // SELL slice offsets [n_slices+1] or CSR row offsets [n+1]
-    const int32_t *swidth = nullptr;     // SELL slice widths (g == 1 only)
-    int32_t wmax = 0;                    // widest SELL slice (g == 1 only)
-    const int32_t *col = nullptr;        // column indices (when col16 is null)
-    const float *val = nullptr;          // FP32 values (when val16 is null)
-    // compressed forms: column = cbase[slice or row] + col16[k]; value =
-    // vscale * half(val16[k]) (IEEE binary16 bits)
-    const uint16_t *col16 = nullptr;
-    const int32_t *cbase = nullptr;
-    const uint16_t *val16 = nullptr;
+    int32_t n = 0;                 // rows
+    int32_t g = 1;                 // lanes per row
+    int32_t c16 = 0;               // 16-bit columns
+    int32_t half = 0;              // binary16 values
     float vscale = 1.0f;
+    int32_t chunks = 0;            // stored chunks
+    // per SELL slice or CSR row its first chunk and its smallest column, and
+    // one closing element: chunk k of SELL row r is head.x + 32 k + (r & 31),
+    // of CSR row r head.x + k
+    const int2 *head = nullptr;
+    // chunks: half and c16: 16 bytes in val, entry j = half << 16 | offset;
+    // else four values in val and four columns in col
+    const void *val = nullptr, *col = nullptr;
 };
 
 constexpr int kAmgMaxLevels = 12;
 
 struct AmgLevelDev {
-    SpOp A;                              // level operator (level 0: the solver's FP32 matrix)
+    SpOp A;                              // level operator (level 0: the solver's FP32 matrix, upload_a0)
     SpOp ST;                             // S^T to the next level, S = (I - omega D^-1 A) P (not on the last two)
     const float *dinv = nullptr;
     float omega = 0.f;
-    float *b = nullptr;                  // right-hand side (levels >= 1)
-    float *t = nullptr;                  // W b
+    float *b = nullptr, *sb = nullptr;   // right-hand side and omega D^-1 b (levels >= 1)
+    float *t = nullptr;                  // W b (levels >= 1)
 };
 
-// The cycle for L = nlev - 1 levels above the coarsest: down-sweep phases
-// t_l = W_l b_l with b_{l+1} = S_l^T b_l, the last one y_L = G b_{L-1}
-// (G = C^-1 S_{L-1}^T); then y_1 = t_1 + U1 [t_2 .. t_{L-1}, y_L] (L >= 2)
-// and z = t_0 + S_0 y_1.  L == 0: z = C^-1 r.
+// The cycle for L = nlev - 1 levels above the coarsest: b_1 = S_0^T r, the
+// down-sweep phases t_l = W_l b_l with b_{l+1} = S_l^T b_l, the last one y_L =
+// G b_{L-1} (G = C^-1 S_{L-1}^T); then y_1 = t_1 + U1 [t_2 .. t_{L-1}, y_L]
+// (L >= 2) and z = W_0 r + S_0 y_1.  L == 0: z = C^-1 r.
 struct AmgDev {
     int32_t nlev = 0;
     AmgLevelDev lev[kAmgMaxLevels];
@@ -300,7 +303,8 @@ struct AmgDev {
     float *stack = nullptr;              // [t_2 .. t_{L-1}, y_L] (L >= 2) or y_1 (L == 1)
     float *yL = nullptr;                 // y_L inside the stack
     float *y1 = nullptr;                 // level-1 result (L >= 2)
-    float *r_alt = nullptr;              // second FP32 residual buffer of the solver [n]
+    float *s0 = nullptr;                 // omega D^-1 r of level 0 [n]
+    const float *diag0 = nullptr;        // diagonal of A_0 [n]
 };
 
 // ---- launch wrappers (all on `stream`) -----------------------------------
