@@ -87,11 +87,11 @@ struct pg_sim {
     double E0_last[3] = {0, 0, 0};
 
     // ESolver (CG1 field): dof -> cell adjacency, cell volumes, mass-matrix
-    // D^-1 (and FP32 values), CG work arrays, the packed vertex field
+    // D^-1 (and FP32 SELL values), work arrays, the packed vertex field
     int64_t *es_adj_ptr = nullptr;
     int32_t *es_adj_cell = nullptr;
     double *es_vol = nullptr, *M_dinv = nullptr, *es_buf = nullptr, *es_part = nullptr, *es_out_d = nullptr;
-    float *M_val32 = nullptr, *M_dinv32 = nullptr, *es_buf32 = nullptr;
+    float *Ms_val32 = nullptr, *M_dinv32 = nullptr, *es_buf32 = nullptr;
     int32_t *es_out_i = nullptr;
     double *Ev = nullptr;
     float *Evf = nullptr;
@@ -1253,6 +1253,10 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
             if ((rc = upload(s, &s->Ms_ptr, mp)) || (rc = upload(s, &s->Ms_width, mw)) ||
                 (rc = upload(s, &s->Ms_col, mc)) || (rc = upload(s, &s->Ms_val, mv)))
                 return bail(rc);
+            if (cfg.precision == PG_MIXED) {
+                std::vector<float> mv32(mv.begin(), mv.end());
+                if ((rc = upload(s, &s->Ms_val32, mv32))) return bail(rc);
+            }
         }
         // SELL-32: slice s holds rows 32s..32s+31 column-major, padded with (row, 0.0)
         const int64_t nsl = (nd + 31) / 32;
@@ -1327,15 +1331,15 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
             return bail(rc);
         cudaMemset(s->Ev, 0, sizeof(double) * 4 * nd);
         if (cfg.precision == PG_MIXED) {
-            std::vector<float> m32(h.M.begin(), h.M.end()), d32(mdinv.begin(), mdinv.end());
-            if ((rc = upload(s, &s->M_val32, m32)) || (rc = upload(s, &s->M_dinv32, d32)) ||
-                (rc = dalloc(s, &s->es_buf32, 18 * nd)) || (rc = dalloc(s, &s->Evf, 4 * nd)))
+            std::vector<float> d32(mdinv.begin(), mdinv.end());
+            if ((rc = upload(s, &s->M_dinv32, d32)) || (rc = dalloc(s, &s->es_buf32, 16 * nd)) ||
+                (rc = dalloc(s, &s->Evf, 4 * nd)))
                 return bail(rc);
-            cudaMemset(s->es_buf32, 0, sizeof(float) * 18 * nd);
+            cudaMemset(s->es_buf32, 0, sizeof(float) * 16 * nd);
             cudaMemset(s->Evf, 0, sizeof(float) * 4 * nd);
         } else {
-            if ((rc = dalloc(s, &s->es_buf, 18 * nd))) return bail(rc);
-            cudaMemset(s->es_buf, 0, sizeof(double) * 18 * nd);
+            if ((rc = dalloc(s, &s->es_buf, 16 * nd))) return bail(rc);
+            cudaMemset(s->es_buf, 0, sizeof(double) * 16 * nd);
         }
         s->dm.Ev = s->Ev;
         s->dm.Evf = s->Evf;
@@ -1667,29 +1671,18 @@ int pg_relocate(pg_sim *s, const double *xs, const int64_t *cells, int64_t n, in
     return PG_OK;
 }
 
-// ESolver::solve (punc/src/efield.cpp:70-75): E = L2 projection of -grad(phi)
-// onto CG1 vector fields, plus the uniform E0, into the packed vertex field.
-// FP64 form: FP64 CG to the reference's tolerances (rel 1e-12, abs 1e-14);
-// mixed form: FP32 CG to rel 1e-6 (the FP32 push reads the field in FP32).
-static int esolver_internal(pg_sim *s, const double E0[3], pg_solve_info *info) {
-    const double zero[3] = {0, 0, 0};
-    launch_efield(s->dm, s->phi, zero, s->stream);
+// The ESolver's arguments: E0 added to the packed field (null: none).  FP64
+// form: the reference's tolerances (rel 1e-12, abs 1e-14); mixed form: FP32 to
+// rel 1e-6 (the FP32 push reads the field in FP32).
+static EsolveArgs esolve_args(pg_sim *s, const double *E0) {
     EsolveArgs e{};
     e.n = s->ndof;
     e.fp32 = is_mixed(s) ? 1 : 0;
     e.adj_ptr = s->es_adj_ptr; e.adj_cell = s->es_adj_cell; e.vol = s->es_vol; e.E_cell = s->dm.E;
-    e.row = s->M_row; e.col = s->M_col; e.val = s->M_val; e.dinv = s->M_dinv;
-    e.val32 = s->M_val32; e.dinv32 = s->M_dinv32;
-    const size_t n3 = 3 * (size_t)s->ndof;
-    if (e.fp32) {
-        float *b = s->es_buf32;
-        e.b32 = b; e.x32 = b + n3; e.r32 = b + 2 * n3; e.z32 = b + 3 * n3; e.p32 = b + 4 * n3; e.Ap32 = b + 5 * n3;
-        e.rtol = 1e-6;
-    } else {
-        double *b = s->es_buf;
-        e.b = b; e.x = b + n3; e.r = b + 2 * n3; e.z = b + 3 * n3; e.p = b + 4 * n3; e.Ap = b + 5 * n3;
-        e.rtol = 1e-12;
-    }
+    e.sptr = s->Ms_ptr; e.swidth = s->Ms_width; e.scol = s->Ms_col; e.sval = s->Ms_val; e.dinv = s->M_dinv;
+    e.sval32 = s->Ms_val32; e.dinv32 = s->M_dinv32;
+    e.buf = s->es_buf; e.buf32 = s->es_buf32;
+    e.rtol = e.fp32 ? 1e-6 : 1e-12;
     e.atol = 1e-14;
     e.max_iter = 1000;
     e.partials = s->es_part;
@@ -1698,6 +1691,15 @@ static int esolver_internal(pg_sim *s, const double E0[3], pg_solve_info *info) 
     for (int j = 0; j < 3; ++j) e.E0[j] = E0 ? E0[j] : 0.0;
     e.ev = s->Ev;
     e.evf = s->Evf;
+    return e;
+}
+
+// ESolver::solve (punc/src/efield.cpp:70-75): E = L2 projection of -grad(phi)
+// onto CG1 vector fields, plus the uniform E0, into the packed vertex field.
+static int esolver_internal(pg_sim *s, const double E0[3], pg_solve_info *info) {
+    const double zero[3] = {0, 0, 0};
+    launch_efield(s->dm, s->phi, zero, s->stream);
+    const EsolveArgs e = esolve_args(s, E0);
     int err;
     {
         StageScope t(s, "efield");
@@ -1715,7 +1717,7 @@ static int esolver_internal(pg_sim *s, const double E0[3], pg_solve_info *info) 
         info->residual = std::sqrt(od[0] + od[1] + od[2]);
         info->rhs_norm = std::sqrt(od[3] + od[4] + od[5]);
     }
-    if (oi[1] != 0) return fail(PG_ERR_NOT_CONVERGED, "ESolver: CG on the mass matrix did not converge");
+    if (oi[1] != 0) return fail(PG_ERR_NOT_CONVERGED, "ESolver: the iteration on the mass matrix did not converge");
     return PG_OK;
 }
 
@@ -2343,32 +2345,9 @@ static int enqueue_step(pg_sim *s, const pg_step_args *a, bool first) {
         if ((rc = pcg_enqueue(s, s->phi))) return rc;
     }
     if (a->efield_cg1) {
-        EsolveArgs e{};
         const double zero[3] = {0, 0, 0};
         launch_efield(s->dm, s->phi, zero, s->stream);
-        e.n = s->ndof;
-        e.fp32 = is_mixed(s) ? 1 : 0;
-        e.adj_ptr = s->es_adj_ptr; e.adj_cell = s->es_adj_cell; e.vol = s->es_vol; e.E_cell = s->dm.E;
-        e.row = s->M_row; e.col = s->M_col; e.val = s->M_val; e.dinv = s->M_dinv;
-        e.val32 = s->M_val32; e.dinv32 = s->M_dinv32;
-        const size_t n3 = 3 * (size_t)s->ndof;
-        if (e.fp32) {
-            float *b = s->es_buf32;
-            e.b32 = b; e.x32 = b + n3; e.r32 = b + 2 * n3; e.z32 = b + 3 * n3; e.p32 = b + 4 * n3; e.Ap32 = b + 5 * n3;
-            e.rtol = 1e-6;
-        } else {
-            double *b = s->es_buf;
-            e.b = b; e.x = b + n3; e.r = b + 2 * n3; e.z = b + 3 * n3; e.p = b + 4 * n3; e.Ap = b + 5 * n3;
-            e.rtol = 1e-12;
-        }
-        e.atol = 1e-14;
-        e.max_iter = 1000;
-        e.partials = s->es_part;
-        e.out_iter = s->es_out_i; e.out_status = s->es_out_i + 1;
-        e.out_rr = s->es_out_d; e.out_bb = s->es_out_d + 3;
-        for (int j = 0; j < 3; ++j) e.E0[j] = a->E0[j];
-        e.ev = s->Ev;
-        e.evf = s->Evf;
+        const EsolveArgs e = esolve_args(s, a->E0);
         const int err = launch_esolve(e, s->stream);
         if (err) return fail(PG_ERR_CUDA, std::string("ESolver launch: ") + cudaGetErrorString((cudaError_t)err));
     } else if (!is_mixed(s)) {

@@ -5,19 +5,29 @@
 // cells T of dof d of (vol_T / 4) (-grad phi_T)_c.
 //
 // The rhs is gathered per dof over its cells in ascending cell order
-// (deterministic).  The three systems are solved together by Jacobi-
-// preconditioned CG in one cooperative launch: one pass over a row of M serves
-// the three components, and the update of A p is folded into the product phase
-// (A p = A z + beta A p_old), so an iteration is two grid barriers.  D^-1 M has
-// its spectrum in [1/2, 5/2] on any P1 tetrahedral mesh (the element mass
-// matrices (vol/20)(I + 1 1^T) scaled by their diagonal), so CG needs ~25
-// iterations for 1e-12.  Arithmetic in T (double for the FP64 form, float for
-// the mixed form); reductions in FP64.
+// (deterministic).  D^-1 M has its spectrum in [1/2, 5/2] on any P1 tetrahedral
+// mesh (the element mass matrices (vol/20)(I + 1 1^T) scaled by their
+// diagonal), so the three systems are solved by Chebyshev iteration on that
+// interval (Golub and Varga 1961): as many products as conjugate gradients
+// need here (30 for 1e-12, 15 for 1e-6 from a cold start), but no inner product
+// in the loop, so one grid barrier per iteration and no reduction, where CG
+// took two barriers and two nine-fold FP64 block and grid sums.  The number
+// of iterations comes from the first residual and the tolerance; the residual
+// is measured then, and again after a few more where it is not met.
+// One pass over a row of M (SELL-32, one thread per row) serves the three
+// components, which are stored together ([n][4]), so an entry costs one gather.
+// One cooperative launch forms the rhs, solves and packs the field.
+// Arithmetic in T (double for the FP64 form, float for the mixed form); the
+// residual's norm in FP64.
+//
+// What bounds it: the chain of loads of a row (entries, then gathers) and the
+// barrier of each iteration; in FP64 also the 45 FP64 operations of a row at
+// 1/64 of the FP32 rate.  Measured against the CG form (GB300, solve with rhs
+// and packing): FP64 9,260 dofs 563 -> 265 us, FP32 39,298 dofs 372 -> 106 us.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "pg_device.cuh"
-#include "pg_reduce.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -27,28 +37,31 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// [n][4] vectors: three components and a pad.
 template <typename T>
-__global__ void k_esolve_rhs(int32_t ndof, const int64_t *__restrict__ adj_ptr, const int32_t *__restrict__ adj_cell,
-                             const double *__restrict__ vol, const double *__restrict__ E, T *__restrict__ b) {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= ndof) return;
-    double bx = 0.0, by = 0.0, bz = 0.0;
-    for (int64_t k = adj_ptr[d]; k < adj_ptr[d + 1]; ++k) {
-        const int c = adj_cell[k];
-        const double w = 0.25 * vol[c];
-        const double2 e01 = __ldg(reinterpret_cast<const double2 *>(E) + 2 * (size_t)c);
-        const double e2 = __ldg(E + 4 * (size_t)c + 2);
-        bx = bx + w * e01.x;
-        by = by + w * e01.y;
-        bz = bz + w * e2;
-    }
-    b[d] = (T)bx;
-    b[ndof + d] = (T)by;
-    b[2 * ndof + d] = (T)bz;
+struct V3 {
+    T x, y, z;
+};
+__device__ __forceinline__ V3<float> load3(const float *p, int i) {
+    const float4 v = reinterpret_cast<const float4 *>(p)[i];
+    return {v.x, v.y, v.z};
+}
+__device__ __forceinline__ V3<double> load3(const double *p, int i) {
+    const double2 *q = reinterpret_cast<const double2 *>(p) + 2 * (size_t)i;
+    const double2 a = q[0];
+    return {a.x, a.y, q[1].x};
+}
+__device__ __forceinline__ void store3(float *p, int i, const V3<float> &v) {
+    reinterpret_cast<float4 *>(p)[i] = make_float4(v.x, v.y, v.z, 0.0f);
+}
+__device__ __forceinline__ void store3(double *p, int i, const V3<double> &v) {
+    double2 *q = reinterpret_cast<double2 *>(p) + 2 * (size_t)i;
+    q[0] = make_double2(v.x, v.y);
+    q[1] = make_double2(v.z, 0.0);
 }
 
-// Sum over the block of N per-thread values; valid in every thread after the
-// call (sh: at least 17 * N doubles).
+// Sums of N per-thread values over the block; valid in thread 0 (sh: 16 N
+// doubles; blocks of at most 16 warps).
 template <int N>
 __device__ __forceinline__ void block_sum_n(const double (&v)[N], double *sh, double (&out)[N]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -56,176 +69,238 @@ __device__ __forceinline__ void block_sum_n(const double (&v)[N], double *sh, do
     for (int k = 0; k < N; ++k) {
         double a = v[k];
         for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) sh[w * N + k] = a;
+        if (lane == 0) sh[k * 16 + w] = a;
     }
     __syncthreads();
-    for (int k = w; k < N; k += nw) {
-        double a = lane < nw ? sh[lane * N + k] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) sh[16 * N + k] = a;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < N; ++k) out[k] = sh[16 * N + k];
-    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 0; k < N; ++k) {
+            double a = 0.0;
+            for (int q = 0; q < nw; ++q) a += sh[k * 16 + q];
+            out[k] = a;
+        }
 }
 
-// Sum of per-block partials part[k * nb + b] over b, for k < N; valid in every
-// thread (one warp per component).
+// Sums over the blocks of part[k * nb + b], k < N, by warp 0; valid in its lane 0.
 template <int N>
-__device__ __forceinline__ void grid_sum_n(const double *part, int nb, double *sh, double (&out)[N]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = w; k < N; k += nw) {
-        double a = 0.0;
-        for (int b = lane; b < nb; b += 32) a += part[k * nb + b];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) sh[k] = a;
-    }
-    __syncthreads();
+__device__ __forceinline__ void grid_sum_n(const double *part, int nb, double (&out)[N]) {
+    if (threadIdx.x >= 32) return;
 #pragma unroll
-    for (int k = 0; k < N; ++k) out[k] = sh[k];
-    __syncthreads();
+    for (int k = 0; k < N; ++k) {
+        double a = 0.0;
+        for (int b = threadIdx.x; b < nb; b += 32) a += __ldcg(part + k * nb + b);
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        out[k] = a;
+    }
 }
+
+// Chebyshev iteration on [1/2, 5/2]: centre, half-width, and -log of its
+// asymptotic rate (acosh(centre / half-width)).  The coefficients converge by a
+// factor of seven per iteration.
+constexpr double kTheta = 1.5, kDelta = 1.0;
+constexpr float kRate = 0.9624237f;
+constexpr int kCheb = 24;
 
 template <typename T>
-struct Cg3Args {
+struct Cheb3Args {
     int32_t n;
-    const int32_t *row, *col;
-    const T *val, *dinv;
-    const T *b;                   // [3][n]
-    T *x, *r, *z, *p, *Ap;        // [3][n]
+    const int64_t *adj_ptr;       // dof -> cells
+    const int32_t *adj_cell;
+    const double *vol, *E_cell;
+    const int64_t *sptr;          // M in SELL-32
+    const int32_t *swidth, *scol;
+    const T *sval, *dinv;
+    T *x, *r, *d0, *d1;           // [n][4]; x: start on entry, solution on return
     double *partials;             // [12][grid]
     double rtol, atol;
     int32_t max_iter;
     int32_t *out_iter, *out_status;
     double *out_rr, *out_bb;      // [3] each
+    double e0[3];
+    double *ev;                   // [n][4] or null
+    float *evf;                   // [n][4] or null
+    T c1[kCheb], c2[kCheb];       // d' = c1 d + c2 D^-1 r of the iterations (the last for all later ones)
 };
 
-// Partials: region A (3 x grid) for p.Ap, region B (9 x grid) for the other
-// sums; alternating regions lets a block write its next partials while slower
-// blocks still read the previous ones, so an iteration needs two barriers.
+// Row i of M times the three components of v.
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 3) k_mass_cg3(Cg3Args<T> a) {
+__device__ __forceinline__ V3<T> mass_row(const Cheb3Args<T> &a, const T *v, int i) {
+    constexpr int C = 4;
+    const int64_t base = __ldg(a.sptr + (i >> 5)) + (i & 31);
+    const int w = __ldg(a.swidth + (i >> 5));
+    V3<T> s{0, 0, 0};
+    for (int k = 0; k < w; k += C) {
+        int c[C];
+        T m[C];
+        V3<T> g[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const bool ok = k + q < w;
+            c[q] = ok ? __ldg(a.scol + base + 32 * (k + q)) : i;
+            m[q] = ok ? __ldg(a.sval + base + 32 * (k + q)) : (T)0;
+        }
+#pragma unroll
+        for (int q = 0; q < C; ++q) g[q] = load3(v, c[q]);
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            s.x += m[q] * g[q].x;
+            s.y += m[q] * g[q].y;
+            s.z += m[q] * g[q].z;
+        }
+    }
+    return s;
+}
+
+// Iterations until ||r||^2 = rr meets tol2 at the asymptotic rate, 1 to 64.
+__device__ __forceinline__ int iterations_left(double rr, double tol2, float slack) {
+    const float ratio2 = (float)(rr / tol2);
+    return max(1, min(64, (int)ceilf((slack + 0.5f * logf(ratio2)) / kRate)));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ Cheb3Args<T> a) {
     cg::grid_group grid = cg::this_grid();
-    __shared__ double sh[17 * 9];
+    __shared__ double sh[16 * 6];
+    __shared__ double tol2[3], rr[3], bb[3];
+    __shared__ int next_check, done, cold[3];
     const int nb = gridDim.x, n = a.n;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gs = nb * blockDim.x;
-    double *partA = a.partials, *partB = a.partials + 3 * nb;
-    const T *val = a.val;
-    // r = b - M x, z = D^-1 r; ||b||^2, r.z, ||r||^2
-    double rz[3], bb[3], rr[3], tol2[3];
+    T *d = a.d0, *dn = a.d1;
+    // b (into dn), r = b - M x, d = D^-1 r / theta
     {
-        double loc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        double loc[6] = {0, 0, 0, 0, 0, 0};
         for (int i = gtid; i < n; i += gs) {
-            T s0 = 0, s1 = 0, s2 = 0;
-            for (int k = a.row[i]; k < a.row[i + 1]; ++k) {
-                const int j = a.col[k];
-                const T v = val[k];
-                s0 += v * a.x[j];
-                s1 += v * a.x[n + j];
-                s2 += v * a.x[2 * n + j];
+            double bx = 0.0, by = 0.0, bz = 0.0;
+            const int64_t k1 = a.adj_ptr[i + 1];
+#pragma unroll 4
+            for (int64_t k = a.adj_ptr[i]; k < k1; ++k) {
+                const int c = __ldg(a.adj_cell + k);
+                const double w = 0.25 * __ldg(a.vol + c);
+                const double2 e01 = __ldg(reinterpret_cast<const double2 *>(a.E_cell) + 2 * (size_t)c);
+                const double e2 = __ldg(a.E_cell + 4 * (size_t)c + 2);
+                bx = bx + w * e01.x;
+                by = by + w * e01.y;
+                bz = bz + w * e2;
             }
-            const T s[3] = {s0, s1, s2};
-            const T di = a.dinv[i];
+            const V3<T> b{(T)bx, (T)by, (T)bz}, s = mass_row(a, a.x, i);
+            const V3<T> r{b.x - s.x, b.y - s.y, b.z - s.z};
+            const T f = a.dinv[i] * (T)(1.0 / kTheta);
+            store3(a.r, i, r);
+            store3(dn, i, b);
+            store3(d, i, V3<T>{f * r.x, f * r.y, f * r.z});
+            loc[0] += (double)r.x * (double)r.x;
+            loc[1] += (double)r.y * (double)r.y;
+            loc[2] += (double)r.z * (double)r.z;
+            loc[3] += (double)b.x * (double)b.x;
+            loc[4] += (double)b.y * (double)b.y;
+            loc[5] += (double)b.z * (double)b.z;
+        }
+        double out[6];
+        block_sum_n<6>(loc, sh, out);
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 6; ++k) a.partials[k * nb + blockIdx.x] = out[k];
+        grid.sync();
+        grid_sum_n<6>(a.partials, nb, out);
+        if (threadIdx.x < 32) {
+            // one lane per component
+            const int c = threadIdx.x;
+            int need = 0;
+            double v = 0.0, u = 0.0;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T bi = a.b[c * n + i];
-                const T ri = bi - s[c];
-                const T zi = di * ri;
-                a.r[c * n + i] = ri;
-                a.z[c * n + i] = zi;
-                loc[c] += (double)bi * (double)bi;
-                loc[3 + c] += (double)ri * (double)zi;
-                loc[6 + c] += (double)ri * (double)ri;
+            for (int q = 0; q < 3; ++q) {
+                const double r0 = __shfl_sync(0xffffffffu, out[q], 0), b0 = __shfl_sync(0xffffffffu, out[3 + q], 0);
+                if (c == q) { v = r0; u = b0; }
+            }
+            if (c < 3) {
+                const double tol = fmax(a.rtol * sqrt(u), a.atol);
+                // a start that is worse than zero is dropped
+                cold[c] = v > u;
+                v = fmin(v, u);
+                rr[c] = v;
+                bb[c] = u;
+                tol2[c] = tol * tol;
+                // 1 / T_k(theta / delta) = 2 exp(-rate k) <= tol / ||r||, and three
+                // iterations more: the error of the slowest modes, which CG
+                // damps below its residual, is then below CG's too (16^3 to
+                // 31^3, CG1 runs: phi within 2e-11 of a 64-bit run, CG 1.1e-10)
+                if (v > tol * tol) need = iterations_left(v, tol * tol, 3.5f);
+            }
+            need = max(need, __shfl_down_sync(0xffffffffu, need, 2));
+            need = max(need, __shfl_down_sync(0xffffffffu, need, 1));
+            if (c == 0) {
+                next_check = min(need, a.max_iter);
+                done = need == 0;
             }
         }
-        double out[9];
-        block_sum_n<9>(loc, sh, out);
-#pragma unroll
-        for (int k = 0; k < 9; ++k)
-            if (threadIdx.x == k) partB[k * nb + blockIdx.x] = out[k];
-        grid.sync();
-        grid_sum_n<9>(partB, nb, sh, out);
-        for (int c = 0; c < 3; ++c) {
-            bb[c] = out[c];
-            rz[c] = out[3 + c];
-            rr[c] = out[6 + c];
-            const double tol = fmax(a.rtol * sqrt(bb[c]), a.atol);
-            tol2[c] = tol * tol;
+        __syncthreads();
+        if (cold[0] || cold[1] || cold[2]) {
+            for (int i = gtid; i < n; i += gs) {
+                const V3<T> b = load3(dn, i);
+                V3<T> x = load3(a.x, i), r = load3(a.r, i), di = load3(d, i);
+                const T f = a.dinv[i] * (T)(1.0 / kTheta);
+                if (cold[0]) { x.x = 0; r.x = b.x; di.x = f * b.x; }
+                if (cold[1]) { x.y = 0; r.y = b.y; di.y = f * b.y; }
+                if (cold[2]) { x.z = 0; r.z = b.z; di.z = f * b.z; }
+                store3(a.x, i, x);
+                store3(a.r, i, r);
+                store3(d, i, di);
+            }
+            grid.sync();
         }
     }
     int it = 0;
-    bool done = rr[0] <= tol2[0] && rr[1] <= tol2[1] && rr[2] <= tol2[2];
-    double beta[3] = {0.0, 0.0, 0.0};
-    bool first = true;
     while (!done && it < a.max_iter) {
-        // A: p = z + beta p, Ap = M z + beta Ap, p.Ap
-        double pap[3] = {0.0, 0.0, 0.0};
-        for (int i = gtid; i < n; i += gs) {
-            T s0 = 0, s1 = 0, s2 = 0;
-            for (int k = a.row[i]; k < a.row[i + 1]; ++k) {
-                const int j = a.col[k];
-                const T v = val[k];
-                s0 += v * a.z[j];
-                s1 += v * a.z[n + j];
-                s2 += v * a.z[2 * n + j];
-            }
-            const T s[3] = {s0, s1, s2};
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T zi = a.z[c * n + i];
-                const T pi = first ? zi : zi + (T)beta[c] * a.p[c * n + i];
-                const T api = first ? s[c] : s[c] + (T)beta[c] * a.Ap[c * n + i];
-                a.p[c * n + i] = pi;
-                a.Ap[c * n + i] = api;
-                pap[c] += (double)pi * (double)api;
-            }
-        }
-        first = false;
-        double alpha[3];
-        {
-            double out[3];
-            block_sum_n<3>(pap, sh, out);
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if (threadIdx.x == k) partA[k * nb + blockIdx.x] = out[k];
-            grid.sync();
-            grid_sum_n<3>(partA, nb, sh, out);
-            for (int c = 0; c < 3; ++c) alpha[c] = (rr[c] > tol2[c] && out[c] > 0.0) ? rz[c] / out[c] : 0.0;
-        }
         ++it;
-        // B: x += alpha p, r -= alpha Ap, z = D^-1 r; r.z, ||r||^2 (rows of this
-        // thread, written in A)
-        double loc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        const bool check = it == next_check;
+        const T c1 = a.c1[min(it, kCheb) - 1], c2 = a.c2[min(it, kCheb) - 1];
+        double *part = a.partials + (size_t)(6 + 3 * (it & 1)) * nb;   // read by all before it is written again
+        double loc[3] = {0, 0, 0};
         for (int i = gtid; i < n; i += gs) {
-            const T di = a.dinv[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T al = (T)alpha[c];
-                a.x[c * n + i] += al * a.p[c * n + i];
-                const T ri = a.r[c * n + i] - al * a.Ap[c * n + i];
-                const T zi = di * ri;
-                a.r[c * n + i] = ri;
-                a.z[c * n + i] = zi;
-                loc[c] += (double)ri * (double)zi;
-                loc[3 + c] += (double)ri * (double)ri;
+            // x += d, r -= M d, d' = c1 d + c2 D^-1 r
+            const V3<T> di = load3(d, i), ri = load3(a.r, i), xi = load3(a.x, i);
+            const T f = c2 * a.dinv[i];
+            const V3<T> s = mass_row(a, d, i);
+            const V3<T> r{ri.x - s.x, ri.y - s.y, ri.z - s.z};
+            store3(a.x, i, V3<T>{xi.x + di.x, xi.y + di.y, xi.z + di.z});
+            store3(a.r, i, r);
+            store3(dn, i, V3<T>{c1 * di.x + f * r.x, c1 * di.y + f * r.y, c1 * di.z + f * r.z});
+            if (check) {
+                loc[0] += (double)r.x * (double)r.x;
+                loc[1] += (double)r.y * (double)r.y;
+                loc[2] += (double)r.z * (double)r.z;
             }
         }
-        {
-            double out[9];
-            block_sum_n<9>(loc, sh, out);
-    #pragma unroll
-        for (int k = 0; k < 9; ++k)
-            if (threadIdx.x == k) partB[k * nb + blockIdx.x] = out[k];
-            grid.sync();
-            grid_sum_n<9>(partB, nb, sh, out);
-            for (int c = 0; c < 3; ++c) {
-                beta[c] = rz[c] > 0.0 ? out[c] / rz[c] : 0.0;
-                rz[c] = out[c];
-                if (rr[c] > tol2[c]) rr[c] = out[3 + c];
-            }
+        T *t = d;
+        d = dn;
+        dn = t;
+        double out[3];
+        if (check) {
+            block_sum_n<3>(loc, sh, out);
+            if (threadIdx.x == 0)
+                for (int k = 0; k < 3; ++k) part[k * nb + blockIdx.x] = out[k];
         }
-        done = rr[0] <= tol2[0] && rr[1] <= tol2[1] && rr[2] <= tol2[2];
+        grid.sync();
+        if (check) {
+            grid_sum_n<3>(part, nb, out);
+            if (threadIdx.x == 0) {
+                int need = 0;
+                for (int c = 0; c < 3; ++c) {
+                    rr[c] = out[c];
+                    if (rr[c] > tol2[c]) need = max(need, iterations_left(rr[c], tol2[c], 0.0f));
+                }
+                done = need == 0;
+                next_check = min(it + need, a.max_iter);
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = gtid; i < n; i += gs) {
+        const V3<T> x = load3(a.x, i);
+        const double ex = (double)x.x + a.e0[0], ey = (double)x.y + a.e0[1], ez = (double)x.z + a.e0[2];
+        if (a.ev) {
+            reinterpret_cast<double2 *>(a.ev)[2 * (size_t)i] = make_double2(ex, ey);
+            reinterpret_cast<double2 *>(a.ev)[2 * (size_t)i + 1] = make_double2(ez, 0.0);
+        }
+        if (a.evf) reinterpret_cast<float4 *>(a.evf)[i] = make_float4((float)ex, (float)ey, (float)ez, 0.0f);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.out_iter = it;
@@ -234,6 +309,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_mass_cg3(Cg3Args<T> a) {
     }
 }
 
+// Planar [3][n] field to the packed vertex field (a field given by the caller).
 template <typename T>
 __global__ void k_pack_ev(int32_t n, const T *__restrict__ x, double e0x, double e0y, double e0z,
                           double *__restrict__ ev, float *__restrict__ evf) {
@@ -247,52 +323,50 @@ __global__ void k_pack_ev(int32_t n, const T *__restrict__ x, double e0x, double
     if (evf) reinterpret_cast<float4 *>(evf)[i] = make_float4((float)ex, (float)ey, (float)ez, 0.0f);
 }
 
+// Blocks of 512 threads, two per SM, or for fewer rows than that blocks of 128,
+// so that the rows spread over the SMs (their FP64 pipes and L1s).
 template <typename T>
-int grid_blocks() {
-    static int g = 0;
-    if (g == 0) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mass_cg3<T>, kThreads, 0);
-        if (per_sm < 1) per_sm = 1;
-        if (per_sm > 3) per_sm = 3;
-        g = per_sm * sm_count();
+void launch_shape(int n, int &blocks, int &threads) {
+    static int per_sm[2] = {0, 0};
+    const int size[2] = {128, 512};
+    for (int k = 0; k < 2; ++k)
+        if (per_sm[k] == 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[k], k_mass_cheb3<T>, size[k], 0);
+            per_sm[k] = per_sm[k] < 1 ? 1 : (per_sm[k] > 2 ? 2 : per_sm[k]);
+        }
+    const int k = (n + size[0] - 1) / size[0] <= per_sm[0] * sm_count() ? 0 : 1;
+    threads = size[k];
+    const int need = (n + threads - 1) / threads, cap = per_sm[k] * sm_count();
+    blocks = need < cap ? need : cap;
+}
+
+template <typename T>
+int solve(const EsolveArgs &e, T *buf, const T *sval, const T *dinv, cudaStream_t st) {
+    const size_t n4 = 4 * (size_t)e.n;
+    Cheb3Args<T> a{e.n, e.adj_ptr, e.adj_cell, e.vol, e.E_cell, e.sptr, e.swidth, e.scol, sval, dinv, buf, buf + n4,
+                   buf + 2 * n4, buf + 3 * n4, e.partials, e.rtol, e.atol, e.max_iter, e.out_iter, e.out_status,
+                   e.out_rr, e.out_bb, {e.E0[0], e.E0[1], e.E0[2]}, e.ev, e.evf, {}, {}};
+    double rho = kDelta / kTheta;
+    for (int k = 0; k < kCheb; ++k) {
+        const double next = 1.0 / (2.0 * kTheta / kDelta - rho);
+        a.c1[k] = (T)(next * rho);
+        a.c2[k] = (T)(2.0 / kDelta * next);
+        rho = next;
     }
-    return g;
+    int blocks = 0, threads = 0;
+    launch_shape<T>(e.n, blocks, threads);
+    void *params[] = {&a};
+    return (int)cudaLaunchCooperativeKernel((const void *)k_mass_cheb3<T>, dim3(blocks), dim3(threads), params, 0, st);
 }
 
 }  // namespace
 
-int esolve_grid_blocks() { return grid_blocks<double>() > grid_blocks<float>() ? grid_blocks<double>() : grid_blocks<float>(); }
+int esolve_grid_blocks() { return 2 * sm_count(); }
 
 int launch_esolve(const EsolveArgs &e, cudaStream_t st) {
-    const int n = e.n;
-    if (n <= 0) return 0;
-    const int blocks = (n + kThreads - 1) / kThreads;
-    count_launches(3);
-    if (e.fp32) {
-        k_esolve_rhs<float><<<blocks, kThreads, 0, st>>>(n, e.adj_ptr, e.adj_cell, e.vol, e.E_cell, e.b32);
-        Cg3Args<float> a{n, e.row, e.col, e.val32, e.dinv32, e.b32, e.x32, e.r32, e.z32, e.p32, e.Ap32,
-                         e.partials, e.rtol, e.atol, e.max_iter, e.out_iter, e.out_status, e.out_rr, e.out_bb};
-        int nb = grid_blocks<float>();
-        if (blocks < nb) nb = blocks;
-        void *params[] = {&a};
-        cudaError_t err = cudaLaunchCooperativeKernel((const void *)k_mass_cg3<float>, dim3(nb), dim3(kThreads), params,
-                                                      0, st);
-        if (err != cudaSuccess) return (int)err;
-        k_pack_ev<float><<<blocks, kThreads, 0, st>>>(n, e.x32, e.E0[0], e.E0[1], e.E0[2], e.ev, e.evf);
-    } else {
-        k_esolve_rhs<double><<<blocks, kThreads, 0, st>>>(n, e.adj_ptr, e.adj_cell, e.vol, e.E_cell, e.b);
-        Cg3Args<double> a{n, e.row, e.col, e.val, e.dinv, e.b, e.x, e.r, e.z, e.p, e.Ap,
-                          e.partials, e.rtol, e.atol, e.max_iter, e.out_iter, e.out_status, e.out_rr, e.out_bb};
-        int nb = grid_blocks<double>();
-        if (blocks < nb) nb = blocks;
-        void *params[] = {&a};
-        cudaError_t err = cudaLaunchCooperativeKernel((const void *)k_mass_cg3<double>, dim3(nb), dim3(kThreads),
-                                                      params, 0, st);
-        if (err != cudaSuccess) return (int)err;
-        k_pack_ev<double><<<blocks, kThreads, 0, st>>>(n, e.x, e.E0[0], e.E0[1], e.E0[2], e.ev, e.evf);
-    }
-    return (int)cudaGetLastError();
+    if (e.n <= 0) return 0;
+    count_launches(1);
+    return e.fp32 ? solve<float>(e, e.buf32, e.sval32, e.dinv32, st) : solve<double>(e, e.buf, e.sval, e.dinv, st);
 }
 
 void launch_pack_ev64(int32_t n, const double *x3, const double E0[3], double *ev, float *evf, cudaStream_t st) {

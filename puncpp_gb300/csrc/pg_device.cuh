@@ -201,8 +201,8 @@ __device__ __forceinline__ float4 dg0_field_f32(const float4 r0, const float4 r1
     return make_float4(__fadd_rn(-gx, e0x), __fadd_rn(-gy, e0y), __fadd_rn(-gz, e0z), 0.0f);
 }
 
-// ESolver: rhs gather, three-component Jacobi-CG on the mass matrix, packing
-// of the vertex field (+ E0).  fp32 selects the FP32 arrays.
+// ESolver: rhs gather, three-component Chebyshev iteration on the mass matrix,
+// packing of the vertex field (+ E0).  fp32 selects the FP32 arrays.
 struct EsolveArgs {
     int32_t n;                    // dofs
     int32_t fp32;
@@ -210,11 +210,12 @@ struct EsolveArgs {
     const int32_t *adj_cell;
     const double *vol;            // [nc]
     const double *E_cell;         // [nc][4], -grad phi per cell
-    const int32_t *row, *col;     // mass matrix CSR
-    const double *val, *dinv;
-    const float *val32, *dinv32;
-    double *b, *x, *r, *z, *p, *Ap;          // [3][n] (FP64 form)
-    float *b32, *x32, *r32, *z32, *p32, *Ap32;  // [3][n] (mixed form)
+    const int64_t *sptr;          // mass matrix in SELL-32
+    const int32_t *swidth, *scol;
+    const double *sval, *dinv;
+    const float *sval32, *dinv32;
+    double *buf;                  // [4][n][4]: x, r, and the two directions (FP64 form)
+    float *buf32;                 // the same (mixed form)
     double *partials;             // [12][grid]
     double rtol, atol;
     int32_t max_iter;
