@@ -29,9 +29,10 @@ struct pg_sim {
 
     // mesh
     DevMesh dm{};
-    int32_t nc = 0, ndof = 0, n_obj = 0, n_ext = 0, n_ofac = 0;
-    std::vector<double> ext_facets_h, obj_facets_h;
-    double *d_ext_facets = nullptr, *d_ofacets = nullptr;
+    int32_t nc = 0, ndof = 0, n_obj = 0, n_ext = 0;
+    std::vector<double> ext_facets_h;
+    double *d_ext_facets = nullptr, *d_ofacets = nullptr;   // object facets sorted by object,
+    int32_t *d_ofac_ptr = nullptr;                          // [n_obj + 1] its offsets
     float4 *d_ext_facets_f = nullptr;     // mixed form: exterior facets in FP32 (InjectParams::facets_f)
 
     // particles (two buffers for the cell sort)
@@ -738,9 +739,6 @@ static int poisson_solve_internal(pg_sim *s, const double *pot_h, bool zero_rho,
                                   double atol, pg_solve_info *acc, double *x_target = nullptr, bool *warm = nullptr) {
     if (s->n_obj > 0) PG_CUDA(cudaMemcpyAsync(s->obj_pot, pot_h, sizeof(double) * s->n_obj, cudaMemcpyHostToDevice, s->stream));
     if (zero_rho) PG_CUDA(cudaMemsetAsync(s->rho_acc, 0, sizeof(double) * s->ndof, s->stream));
-    launch_rhs(s->dm, s->Ms_ptr, s->Ms_width, s->Ms_col, s->Ms_val, zero_rho ? s->rho_acc : s->rho, s->bc_kind, s->bc_value, s->w_ext,
-               s->w_obj, s->obj_pot, s->n_obj, use_ext ? 1 : 0, s->b, s->stream);
-    if (zero_rho) s->rho_valid = false;
     double *x = x_target ? x_target : s->phi;
     bool *valid = warm ? warm : &s->phi_valid;
     if (!(s->cfg.pcg_warm_start && *valid) || zero_rho) {
@@ -757,7 +755,10 @@ static int poisson_solve_internal(pg_sim *s, const double *pot_h, bool zero_rho,
         else PG_CUDA(cudaMemcpyAsync(s->x_prev, x, sizeof(double) * s->ndof, cudaMemcpyDeviceToDevice, s->stream));
         ++s->x_prev_count;
     }
-    launch_set_bc(s->bc_kind, use_ext ? s->bc_value : nullptr, s->obj_pot, s->ndof, x, s->stream);
+    launch_rhs(s->dm, s->Ms_ptr, s->Ms_width, s->Ms_col, s->Ms_val, zero_rho ? s->rho_acc : s->rho, s->bc_kind, s->bc_value, s->w_ext,
+               s->w_obj, s->obj_pot, std::any_of(pot_h, pot_h + s->n_obj, [](double v) { return v != 0.0; }) ? s->n_obj : 0,
+               use_ext ? 1 : 0, s->b, x, s->stream);
+    if (zero_rho) s->rho_valid = false;
     PcgArgs a{};
     a.n = s->ndof;
     a.slice_ptr = s->A_sptr; a.slice_width = s->A_swidth; a.col = s->A_col; a.val = s->A_val; a.dinv = s->A_dinv;
@@ -801,7 +802,7 @@ static int poisson_solve_internal(pg_sim *s, const double *pot_h, bool zero_rho,
 static int image_charges(pg_sim *s, std::vector<double> &out, const double *phi = nullptr) {
     out.assign(s->n_obj, 0.0);
     if (s->n_obj == 0) return PG_OK;
-    launch_image_charge(s->dm, phi ? phi : s->phi, s->d_ofacets, s->n_ofac, s->n_obj, s->cfg.eps0, s->image, s->stream);
+    launch_image_charge(s->dm, phi ? phi : s->phi, s->d_ofacets, s->d_ofac_ptr, s->n_obj, s->cfg.eps0, s->image, s->stream);
     PG_CUDA(cudaMemcpyAsync(out.data(), s->image, sizeof(double) * s->n_obj, cudaMemcpyDeviceToHost, s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
     return PG_OK;
@@ -1047,7 +1048,6 @@ static int inject_internal(pg_sim *s, double dt, uint64_t seed, uint64_t step, b
         const double unit = fixed_unit(s);
         for (int k = 0; k < s->n_species; ++k) ipd.q_scaled[k] = (float)(s->q[k] / unit);
     }
-    PG_CUDA(cudaMemsetAsync(s->inj_counts, 0, sizeof(int64_t) * (total + 1), s->stream));
     PG_CUDA(cudaMemsetAsync(s->state->injected, 0, sizeof(s->state->injected), s->stream));
     launch_inject_count(s->dm, ipd, s->flux_num, s->inj_counts, s->stream);
     launch_scan_i64(s->inj_counts, s->inj_offsets, total + 1, s->scan_tmp, s->stream);
@@ -1347,10 +1347,20 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
 
     // boundary facets
     s->ext_facets_h = h.ext_facets;
-    s->obj_facets_h = h.obj_facets;
     s->n_ext = (int32_t)(h.ext_facets.size() / 14);
-    s->n_ofac = (int32_t)(h.obj_facets.size() / 7);
-    if ((rc = upload(s, &s->d_ext_facets, h.ext_facets)) || (rc = upload(s, &s->d_ofacets, h.obj_facets))) return bail(rc);
+    {
+        const size_t nf = h.obj_facets.size() / 7;
+        std::vector<int32_t> ptr(s->n_obj + 1, 0);
+        std::vector<double> sorted(h.obj_facets.size());
+        for (size_t f = 0; f < nf; ++f) ++ptr[(size_t)h.obj_facets[7 * f + 1] + 1];
+        for (int32_t o = 0; o < s->n_obj; ++o) ptr[o + 1] += ptr[o];
+        std::vector<int32_t> at(ptr.begin(), ptr.end());
+        for (size_t f = 0; f < nf; ++f)
+            std::copy_n(&h.obj_facets[7 * f], 7, &sorted[7 * (size_t)at[(size_t)h.obj_facets[7 * f + 1]]++]);
+        if ((rc = upload(s, &s->d_ext_facets, h.ext_facets)) || (rc = upload(s, &s->d_ofacets, sorted)) ||
+            (rc = upload(s, &s->d_ofac_ptr, ptr)))
+            return bail(rc);
+    }
     if (cfg.precision == PG_MIXED && s->n_ext > 0) {
         std::vector<float4> ff(4 * (size_t)s->n_ext);
         for (int64_t j = 0; j < s->n_ext; ++j) {
@@ -2251,11 +2261,11 @@ int pg_sort(pg_sim *s) {
 // ---- multi-step runs: the step on the device only ------------------------
 
 // rhs, boundary values and one PCG launch into x; object potentials are read
-// from s->obj_pot on the device; no status read-back.
-static int pcg_enqueue(pg_sim *s, double *x) {
+// from s->obj_pot on the device (zero_pot: all of them zero there); no status
+// read-back.
+static int pcg_enqueue(pg_sim *s, double *x, bool zero_pot) {
     launch_rhs(s->dm, s->Ms_ptr, s->Ms_width, s->Ms_col, s->Ms_val, s->rho, s->bc_kind, s->bc_value, s->w_ext, s->w_obj, s->obj_pot,
-               s->n_obj, 1, s->b, s->stream);
-    launch_set_bc(s->bc_kind, s->bc_value, s->obj_pot, s->ndof, x, s->stream);
+               zero_pot ? 0 : s->n_obj, 1, s->b, x, s->stream);
     PcgArgs a{};
     a.n = s->ndof;
     a.slice_ptr = s->A_sptr; a.slice_width = s->A_swidth; a.col = s->A_col; a.val = s->A_val; a.dinv = s->A_dinv;
@@ -2315,13 +2325,10 @@ static void inject_enqueue(pg_sim *s, const DevParticles &Pd, double dt, uint64_
     ip.rho_fixed = s->rho_fixed;
     const double unit = fixed_unit(s);
     for (int k = 0; k < s->n_species; ++k) ip.q_scaled[k] = (float)(s->q[k] / unit);
-    cudaMemsetAsync(s->inj_counts, 0, sizeof(int64_t) * (total + 1), s->stream);
-    cudaMemsetAsync(s->state->injected, 0, sizeof(s->state->injected), s->stream);
     launch_inject_count(s->dm, ip, s->flux_num, s->inj_counts, s->stream);
     launch_scan_i64(s->inj_counts, s->inj_offsets, total + 1, s->scan_tmp, s->stream);
     launch_inject_generate(s->dm, Pd, ip, s->flux_num, s->pdf_max, s->d_ext_facets, s->inj_offsets,
                            s->cfg.max_walk_steps, 1, s->d_q, s->rho_acc, s->state, inject_bound(s, dt), s->stream);
-    launch_inject_commit(s->run_counts, s->state, s->stream);
 }
 
 // One whole step on the stream, no host synchronisation: the same operations
@@ -2335,14 +2342,14 @@ static int enqueue_step(pg_sim *s, const pg_step_args *a, bool first) {
     if (s->circuit_ready) {
         launch_circuit_pre(s->run_isrc, (int)s->isrc.size(), s->circ_dt, s->n_obj, s->run_obj, s->obj_pot, s->stream);
         const bool superpose = !s->cfg.circuit_resolve && s->lap;
-        if ((rc = pcg_enqueue(s, superpose ? s->phi0 : s->phi))) return rc;
-        launch_image_charge(s->dm, superpose ? s->phi0 : s->phi, s->d_ofacets, s->n_ofac, s->n_obj, s->cfg.eps0,
+        if ((rc = pcg_enqueue(s, superpose ? s->phi0 : s->phi, true))) return rc;
+        launch_image_charge(s->dm, superpose ? s->phi0 : s->phi, s->d_ofacets, s->d_ofac_ptr, s->n_obj, s->cfg.eps0,
                             s->image, s->stream);
         launch_circuit_post(s->circ_dev, s->image, s->run_obj, s->obj_pot, s->stream);
         if (superpose) launch_superpose_dev(s->phi0, s->lap, s->obj_pot, s->lap_rng, s->n_obj, s->ndof, s->phi, s->stream);
-        else if ((rc = pcg_enqueue(s, s->phi))) return rc;
+        else if ((rc = pcg_enqueue(s, s->phi, false))) return rc;
     } else {
-        if ((rc = pcg_enqueue(s, s->phi))) return rc;
+        if ((rc = pcg_enqueue(s, s->phi, false))) return rc;
     }
     if (a->efield_cg1) {
         const double zero[3] = {0, 0, 0};
@@ -2354,7 +2361,8 @@ static int enqueue_step(pg_sim *s, const pg_step_args *a, bool first) {
         step_field_f64(s, a->E0);
     }
     const double dt_push = first ? 0.5 * a->dt : a->dt;
-    cudaMemsetAsync(s->state->absorbed, 0, sizeof(s->state->absorbed), s->stream);
+    // absorbed and injected, one after the other in DevState
+    cudaMemsetAsync(s->state->absorbed, 0, sizeof(s->state->absorbed) + sizeof(s->state->injected), s->stream);
     if (is_mixed(s)) {
         cudaMemsetAsync(s->rho_fixed, 0, sizeof(unsigned long long) * s->ndof, s->stream);
         MixedParams xp;
@@ -2375,11 +2383,10 @@ static int enqueue_step(pg_sim *s, const pg_step_args *a, bool first) {
         launch_fused_step(s->dm, Pd, cap, pp, mp, s->cfg.max_walk_steps, s->d_q, s->rho_acc, s->state, s->partials,
                           s->n_part, s->ke_dev, s->stream);
     }
-    launch_objects_update(s->state, s->d_q, s->n_species, s->run_tags, s->n_obj, s->run_obj, a->dt, s->stream);
     if (a->inject) inject_enqueue(s, Pd, a->dt, a->seed);
-    else cudaMemsetAsync(s->state->injected, 0, sizeof(s->state->injected), s->stream);
-    launch_step_record(s->run_rows, 6 + 3 * s->n_obj, s->run_counts, s->ke_dev, s->state, s->n_species, s->pcg_out_i,
-                       s->pcg_out_d, s->run_obj, s->n_obj, s->stream);
+    launch_step_finish(s->run_rows, 6 + 3 * s->n_obj, s->run_counts, s->ke_dev, s->state, s->d_q, s->n_species,
+                       a->inject && s->n_inj_species * s->n_ext > 0 ? 1 : 0, s->pcg_out_i, s->pcg_out_d, s->run_tags,
+                       s->run_obj, s->n_obj, a->dt, s->stream);
     return PG_OK;
 }
 
@@ -2423,6 +2430,10 @@ static int upload_circuit(pg_sim *s) {
     c.n_groups = (int32_t)s->groups.size();
     c.n_fv = (int32_t)s->fixed_voltage.size();
     c.g_ptr = d_gp; c.g_mem = d_gm; c.f_ptr = d_fp; c.f_mem = d_fm;
+    std::vector<int32_t> members(gm);
+    members.insert(members.end(), fm.begin(), fm.end());
+    std::sort(members.begin(), members.end());
+    c.distinct = std::adjacent_find(members.begin(), members.end()) == members.end() ? 1 : 0;
     c.inv_cap = d_ic; c.inv_circ = d_icc; c.cv = d_cv;
     std::vector<double> isrc;
     for (auto &x : s->isrc) { isrc.push_back(x.node_a); isrc.push_back(x.node_b); isrc.push_back(x.value); }

@@ -49,6 +49,7 @@ __device__ __forceinline__ void uniforms2(uint64_t seed, uint32_t block, uint32_
 
 __global__ void k_inject_count(InjectParams ip, const double *__restrict__ flux_num, int64_t *__restrict__ counts) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx == ip.n_species * ip.n_facets) counts[idx] = 0;   // the scan's total
     if (idx >= ip.n_species * ip.n_facets) return;
     const int s = idx / ip.n_facets, j = idx % ip.n_facets;
     const double nf = flux_num[idx] * ip.sp[s].ndt;
@@ -255,7 +256,7 @@ void launch_inject_count(const DevMesh &m, const InjectParams &ip, const double 
     const int total = ip.n_species * ip.n_facets;
     if (total <= 0) return;
     count_launches(1);
-    k_inject_count<<<(total + kThreads - 1) / kThreads, kThreads, 0, st>>>(ip, flux_num, counts);
+    k_inject_count<<<total / kThreads + 1, kThreads, 0, st>>>(ip, flux_num, counts);
 }
 
 void launch_inject_generate(const DevMesh &m, const DevParticles &p, const InjectParams &ip, const double *flux_num,

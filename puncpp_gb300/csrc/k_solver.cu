@@ -32,35 +32,52 @@ __global__ void k_efield(DevMesh m, const double *__restrict__ phi, double e0x, 
 
 // b = M rho on free rows, minus the Dirichlet columns moved to the right-hand
 // side; b = g on Dirichlet rows (PoissonSolver::solve, punc/src/poisson.cpp:343-362,
-// with the BC rows eliminated symmetrically).  M in SELL-32 (one thread per
-// row, the row's entries in their CSR order; padding: value 0, own column).
-__global__ void k_rhs(int32_t n, const int64_t *__restrict__ sptr, const int32_t *__restrict__ swidth,
-                      const int32_t *__restrict__ scol, const double *__restrict__ sval,
-                      const double *__restrict__ rho, const int32_t *__restrict__ bc_kind,
-                      const double *__restrict__ bc_value, const double *__restrict__ w_ext,
-                      const double *__restrict__ w_obj, const double *__restrict__ obj_pot, int32_t n_obj,
-                      int32_t use_ext, double *__restrict__ b) {
+// with the BC rows eliminated symmetrically), which the start x of the solve
+// takes too.  M in SELL-32 (one thread per row, the row's entries in their CSR
+// order; padding: value 0, own column).  n_w: the objects' columns to subtract
+// (0 when every object potential is zero).  Bound by HBM at 12 bytes an entry
+// and by the FP64 pipe at two operations an entry, so one fused operation each,
+// five entries' loads together (531k rows, 7.8M entries: 41 -> 26 us), and by
+// w_obj at many objects (24 of them, 122k rows: 28 us).
+__global__ void __launch_bounds__(kThreads) k_rhs(int32_t n, const int64_t *__restrict__ sptr,
+                                                  const int32_t *__restrict__ swidth, const int32_t *__restrict__ scol,
+                                                  const double *__restrict__ sval, const double *__restrict__ rho,
+                                                  const int32_t *__restrict__ bc_kind,
+                                                  const double *__restrict__ bc_value, const double *__restrict__ w_ext,
+                                                  const double *__restrict__ w_obj, const double *__restrict__ obj_pot,
+                                                  int32_t n_w, int32_t use_ext, double *__restrict__ b,
+                                                  double *__restrict__ x) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int k = bc_kind[i];
-    if (k == 0) { b[i] = use_ext ? bc_value[i] : 0.0; return; }
-    if (k > 0) { b[i] = obj_pot[k - 1]; return; }
+    if (k >= 0) {
+        const double g = k > 0 ? obj_pot[k - 1] : (use_ext ? bc_value[i] : 0.0);
+        b[i] = g;
+        x[i] = g;
+        return;
+    }
     const int64_t base = __ldg(sptr + (i >> 5)) + (i & 31);
     const int w = __ldg(swidth + (i >> 5));
     double s = 0.0;
-    for (int e = 0; e < w; ++e) s += __ldg(sval + base + 32 * e) * __ldg(rho + __ldg(scol + base + 32 * e));
+    constexpr int C = 5;
+    for (int e = 0; e < w; e += C) {
+        int c[C];
+        double v[C], r[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const bool ok = e + q < w;
+            c[q] = ok ? __ldg(scol + base + 32 * (e + q)) : i;
+            v[q] = ok ? __ldg(sval + base + 32 * (e + q)) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < C; ++q) r[q] = __ldg(rho + c[q]);
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+            if (e + q < w) s = fma(v[q], r[q], s);
+    }
     if (use_ext) s = s - w_ext[i];
-    for (int o = 0; o < n_obj; ++o) s = s - obj_pot[o] * w_obj[(size_t)o * n + i];
+    for (int o = 0; o < n_w; ++o) s = s - obj_pot[o] * w_obj[(size_t)o * n + i];
     b[i] = s;
-}
-
-__global__ void k_set_bc(const int32_t *__restrict__ bc_kind, const double *__restrict__ bc_value,
-                         const double *__restrict__ obj_pot, int32_t n, double *__restrict__ x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int k = bc_kind[i];
-    if (k == 0) x[i] = bc_value ? bc_value[i] : 0.0;
-    else if (k > 0) x[i] = obj_pot[k - 1];
 }
 
 // Sum of one value per block, then every block reads all block partials in
@@ -406,30 +423,31 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_rel(PcgArgs a) {
 
 // Image charge of each object: sum over its facets of
 // eps0 * area * grad(phi_T) . n (the Charge.ufl ds-integral for P1,
-// CircuitCM::post_solve, punc/src/object_CM.cpp:328-337).  One block, facets
-// in list order, per-object partial sums combined in a fixed tree order.
-__global__ void k_image_charge(DevMesh m, const double *__restrict__ phi, const double *__restrict__ of, int32_t nf,
-                               int32_t n_obj, double eps0, double *__restrict__ out) {
+// CircuitCM::post_solve, punc/src/object_CM.cpp:328-337).  One block per object
+// over its own facets (list order, sorted by object: ptr), partial sums
+// combined in a fixed tree order.  Latency-bound (facet, dofs, potentials);
+// with one block that went through all facets for each object, 24 objects took
+// 151 us, now 7.
+__global__ void k_image_charge(DevMesh m, const double *__restrict__ phi, const double *__restrict__ of,
+                               const int32_t *__restrict__ ptr, double eps0, double *__restrict__ out) {
     __shared__ double sh[32];
-    for (int o = 0; o < n_obj; ++o) {
-        double v = 0.0;
-        for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-            const double *r = of + 7 * (size_t)f;
-            if ((int)r[1] != o) continue;
-            const int c = (int)r[0];
-            const int4 d = m.dofs[c];
-            const double p3 = phi[d.w];
-            const double a = phi[d.x] - p3, b = phi[d.y] - p3, e = phi[d.z] - p3;
-            const double *A = m.bary + 12 * (size_t)c;
-            const double gx = a * A[1] + b * A[5] + e * A[9];
-            const double gy = a * A[2] + b * A[6] + e * A[10];
-            const double gz = a * A[3] + b * A[7] + e * A[11];
-            const double gn = gx * r[3] + gy * r[4] + gz * r[5];
-            v += (eps0 * r[2]) * gn;
-        }
-        v = block_reduce(v, sh);
-        if (threadIdx.x == 0) out[o] = v;
+    const int o = blockIdx.x;
+    double v = 0.0;
+    for (int f = ptr[o] + threadIdx.x; f < ptr[o + 1]; f += blockDim.x) {
+        const double *r = of + 7 * (size_t)f;
+        const int c = (int)r[0];
+        const int4 d = m.dofs[c];
+        const double p3 = phi[d.w];
+        const double a = phi[d.x] - p3, b = phi[d.y] - p3, e = phi[d.z] - p3;
+        const double *A = m.bary + 12 * (size_t)c;
+        const double gx = a * A[1] + b * A[5] + e * A[9];
+        const double gy = a * A[2] + b * A[6] + e * A[10];
+        const double gz = a * A[3] + b * A[7] + e * A[11];
+        const double gn = gx * r[3] + gy * r[4] + gz * r[5];
+        v += (eps0 * r[2]) * gn;
     }
+    v = block_reduce(v, sh);
+    if (threadIdx.x == 0) out[o] = v;
 }
 
 // phi = phi0 + sum_k V_k L_k: the solution with object potentials V from the
@@ -460,17 +478,11 @@ void launch_efield(const DevMesh &m, const double *phi, const double E0[3], cuda
 
 void launch_rhs(const DevMesh &m, const int64_t *msptr, const int32_t *mswidth, const int32_t *mscol,
                 const double *msval, const double *rho, const int32_t *bc_kind, const double *bc_value,
-                const double *w_ext, const double *w_obj, const double *obj_pot, int32_t n_obj, int32_t use_ext,
-                double *b, cudaStream_t st) {
+                const double *w_ext, const double *w_obj, const double *obj_pot, int32_t n_w, int32_t use_ext,
+                double *b, double *x, cudaStream_t st) {
     count_launches(1);
     k_rhs<<<(m.ndof + kThreads - 1) / kThreads, kThreads, 0, st>>>(m.ndof, msptr, mswidth, mscol, msval, rho, bc_kind,
-                                                                    bc_value, w_ext, w_obj, obj_pot, n_obj, use_ext, b);
-}
-
-void launch_set_bc(const int32_t *bc_kind, const double *bc_value, const double *obj_pot, int32_t n, double *x,
-                   cudaStream_t st) {
-    count_launches(1);
-    k_set_bc<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(bc_kind, bc_value, obj_pot, n, x);
+                                                                    bc_value, w_ext, w_obj, obj_pot, n_w, use_ext, b, x);
 }
 
 int pcg_grid_blocks() {
@@ -499,11 +511,11 @@ int launch_pcg(const PcgArgs &a, cudaStream_t st) {
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-void launch_image_charge(const DevMesh &m, const double *phi, const double *ofacets, int32_t n_ofacets, int32_t n_obj,
+void launch_image_charge(const DevMesh &m, const double *phi, const double *ofacets, const int32_t *ptr, int32_t n_obj,
                          double eps0, double *out, cudaStream_t st) {
     if (n_obj <= 0) return;
     count_launches(1);
-    k_image_charge<<<1, 1024, 0, st>>>(m, phi, ofacets, n_ofacets, n_obj, eps0, out);
+    k_image_charge<<<n_obj, 512, 0, st>>>(m, phi, ofacets, ptr, eps0, out);
 }
 
 }  // namespace pg

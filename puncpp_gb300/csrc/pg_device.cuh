@@ -348,10 +348,8 @@ void launch_sort_scatter(const DevParticles &src, const DevParticles &dst, int64
 
 void launch_rhs(const DevMesh &m, const int64_t *msptr, const int32_t *mswidth, const int32_t *mscol,
                 const double *msval, const double *rho, const int32_t *bc_kind, const double *bc_value,
-                const double *w_ext, const double *w_obj, const double *obj_pot, int32_t n_obj, int32_t use_ext,
-                double *b, cudaStream_t st);
-void launch_set_bc(const int32_t *bc_kind, const double *bc_value, const double *obj_pot,
-                   int32_t n, double *x, cudaStream_t st);
+                const double *w_ext, const double *w_obj, const double *obj_pot, int32_t n_w, int32_t use_ext,
+                double *b, double *x, cudaStream_t st);
 int launch_pcg(const PcgArgs &a, cudaStream_t st);
 int pcg_grid_blocks();
 int launch_pcg_amg(const PcgArgs &a, const AmgDev &amg, cudaStream_t st);
@@ -386,18 +384,16 @@ struct CircuitDev {
     const double *inv_cap = nullptr;     // [n][n]
     const double *inv_circ = nullptr;    // [2n][2n]
     double *cv = nullptr;                // [2n] circuit vector
+    int32_t distinct = 0;                // no object is in two groups or fixed-voltage sets
 };
-void launch_inject_commit(int64_t *counts, const DevState *st, cudaStream_t s);
-void launch_objects_update(const DevState *st, const double *q, int n_species, const int64_t *tags, int n_obj,
-                           double *obj, double dt, cudaStream_t s);
 void launch_circuit_pre(const double *isrc, int n_isrc, double circ_dt, int n_obj, double *obj, double *obj_pot,
                         cudaStream_t s);
 void launch_circuit_post(const CircuitDev &c, const double *img, double *obj, double *obj_pot, cudaStream_t s);
 void launch_superpose_dev(const double *phi0, const double *lap, const double *pot, const int32_t *rng, int n_obj,
                          int32_t n, double *out, cudaStream_t s);
-void launch_step_record(double *rows, int row_len, int64_t *counts, const double *ke, const DevState *st,
-                        int n_species, const int32_t *pcg_i, const double *pcg_d, const double *obj, int n_obj,
-                        cudaStream_t s);
+void launch_step_finish(double *rows, int row_len, int64_t *counts, const double *ke, const DevState *st, const double *q,
+                        int n_species, int injected, const int32_t *pcg_i, const double *pcg_d, const int64_t *tags,
+                        double *obj, int n_obj, double dt, cudaStream_t s);
 void launch_set_count(int64_t *counts, const int64_t *cursor, int32_t nc, cudaStream_t s);
 
 // adjoint of the fused steps (k_adjoint.cu)
@@ -426,7 +422,7 @@ void launch_fixed_to_rho(const unsigned long long *fixed, const double *dv_inv, 
                          double *rho_acc, double *rho, cudaStream_t st);
 void launch_float_tables(const double *bary, const double *planes, const int4 *nbr, int32_t nc, double X,
                          float4 *cell_f, float *lam_abs, cudaStream_t st);
-void launch_image_charge(const DevMesh &m, const double *phi, const double *ofacets, int32_t n_ofacets,
-                         int32_t n_obj, double eps0, double *out, cudaStream_t st);
+void launch_image_charge(const DevMesh &m, const double *phi, const double *ofacets, const int32_t *ptr, int32_t n_obj,
+                         double eps0, double *out, cudaStream_t st);
 
 }  // namespace pg
