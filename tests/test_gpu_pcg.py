@@ -1,6 +1,7 @@
 """The AMG-PCG solve against a direct solve on hierarchies of one level (the
 dense inverse), two and three, operators in natural and random order, systems
-of one block and of many, row counts that are no multiple of a slice."""
+of one block, of a cluster (up to 16,384 rows) and of a grid, row counts that are
+no multiple of a slice."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
