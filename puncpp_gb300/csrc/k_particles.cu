@@ -45,6 +45,14 @@ __device__ __forceinline__ bool inside_fp64(const DevMesh &m, double x, double y
 }
 
 // One pass over the particle slots doing any of push, move, walk and deposit.
+// Bound by the FP64 pipe (about 47 operations a particle, none contracted
+// where the reference's bits count).  The lanes of a warp take their 32 slots
+// together and meet again before and after the walk, whose lanes end in
+// different iterations: left to run on apart, 18 of 32 lanes were active in
+// an average instruction, and every FP64 operation of a part of a warp costs
+// as much as that of a whole one (53^3 cells, 1.5M particles: 224 -> 153 us, of
+// which 112 are the FP64 operations at full rate; the mixed form's pass, bound
+// by loads, does not change with it).
 template <bool PUSH, bool HAS_B, bool ACCEL, bool MOVE, bool PERIODIC, bool WALK, bool DEPOSIT>
 __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, int64_t n_slots, PushParams pp,
                                                        MoveParams mp, int max_steps, const double *__restrict__ qsp,
@@ -53,12 +61,15 @@ __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, in
     double ke = 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t n_use = slots_in_use(p, n_slots);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_use; i += stride) {
-        int c = p.cell[i];
-        if (c < 0) continue;
-        const int s = p.sp[i];
-        double x = p.x[i], y = p.y[i], z = p.z[i];
-        if (PUSH || MOVE) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < n_use; base += stride) {
+        const int64_t i = base + lane;
+        int c = i < n_use ? p.cell[i] : kDead;
+        bool live = c >= 0;
+        int s = 0;
+        double x = 0.0, y = 0.0, z = 0.0;
+        if (live) { s = p.sp[i]; x = p.x[i]; y = p.y[i]; z = p.z[i]; }
+        if ((PUSH || MOVE) && live) {
             double vx = p.vx[i], vy = p.vy[i], vz = p.vz[i];
             if (PUSH) {
                 double ex, ey, ez;
@@ -122,23 +133,26 @@ __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, in
                 p.x[i] = x; p.y[i] = y; p.z[i] = z;
             }
         }
-        if (WALK) {
+        if (WALK) __syncwarp();
+        if (WALK && live) {
             // Population::update (punc/include/punc/population.h:641-699).
             const int nc = walk_fp64<PERIODIC || !MOVE>(m, x, y, z, c, max_steps);
             if (nc == kWalkFail) {
                 raise_device_error(st, PG_ERR_WALK_LIMIT, i);
-                continue;
-            }
-            if (nc < 0) {
+                live = false;
+            } else if (nc < 0) {
                 const int tag = -nc;
                 atomicAdd(reinterpret_cast<unsigned long long *>(&st->absorbed[tag < kMaxTags ? tag : 0][s]), 1ull);
                 atomicAdd(reinterpret_cast<unsigned long long *>(&st->live[s]), ~0ull);
                 p.cell[i] = kDead;
-                continue;
+                live = false;
+            } else if (nc != c) {
+                p.cell[i] = nc;
+                c = nc;
             }
-            if (nc != c) { p.cell[i] = nc; c = nc; }
         }
-        if (DEPOSIT) {
+        if (WALK) __syncwarp();
+        if (DEPOSIT && live) {
             // distribute_cg1 (punc/include/punc/distributor.h:168-210): q * lambda_i.
             double l0, l1, l2, l3;
             barycentric_fp64(m, c, x, y, z, l0, l1, l2, l3);

@@ -97,7 +97,7 @@ constexpr int kNearSteps = 256;
 // point (T: double or float).  One 64-byte record per cell visited instead of
 // 144 bytes, and no FP64 operation outside the bound (a plane test is six, at
 // 1/64 of the FP32 rate; the FP64 pass over 1.5M particles at 53^3 cells 525
-// us with them, 224 without).  R, have_rec: the first cell's record when the
+// us with them, 224 without, then 153 with the warp kept together).  R, have_rec: the first cell's record when the
 // caller has it; R and l are the last cell's on return.
 //
 // NEAR: in a mesh whose cells fill their bounding box (m.box; set only with a
