@@ -83,7 +83,7 @@ __device__ __forceinline__ DF df_mul(DF a, float b) {
 constexpr int kWarps = kPcgThreads / 32;
 
 // The barrier between phases: of a cooperative grid, or of one thread-block
-// cluster (the hardware's).
+// cluster (the hardware's; all threads of a warp arrive together).
 struct GridSync {
     static constexpr bool kCluster = false;
     __device__ __forceinline__ static void sync() { cg::this_grid().sync(); }
@@ -91,7 +91,8 @@ struct GridSync {
 struct ClusterSync {
     static constexpr bool kCluster = true;
     __device__ __forceinline__ static void sync() {
-        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 };
 constexpr int kClusterMax = 16;   // blocks of a cluster
@@ -108,6 +109,11 @@ __device__ __forceinline__ void store_remote(DF *p, DF v, int rank) {
 // one thread's store to part[q * nb + blockIdx.x] in global memory, or in a
 // cluster to part[q * kClusterMax + blockIdx.x] in every block's shared memory
 // (read there without a trip to the L2).  sh: kWarps * K values.
+//
+// Every warp runs the shuffles of both functions, though K of them suffice: a
+// shuffle where the warp may have diverged (under a test of the warp's number,
+// or after loads by a part of the lanes) took 250 cycles instead of 25, and a
+// total 1.3 us (cluster) to 2.6 (77 blocks) instead of 0.3 to 0.8.
 template <int K, class Sync>
 __device__ __forceinline__ void block_part(DF (&v)[K], DF *sh, DF *part, int nb) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -118,16 +124,13 @@ __device__ __forceinline__ void block_part(DF (&v)[K], DF *sh, DF *part, int nb)
         if (lane == 0) sh[q * kWarps + w] = v[q];
     }
     __syncthreads();
-    if (w < K) {
-        DF s = lane < kWarps ? sh[w * kWarps + lane] : DF{0.0f, 0.0f};
-        for (int o = kWarps / 2; o > 0; o >>= 1)
-            s = df_add(s, DF{__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.lo, o)});
-        if (Sync::kCluster) {
-            s = DF{__shfl_sync(0xffffffffu, s.hi, 0), __shfl_sync(0xffffffffu, s.lo, 0)};
-            if (lane < nb) store_remote(part + w * kClusterMax + blockIdx.x, s, lane);
-        } else if (lane == 0) {
-            part[w * nb + blockIdx.x] = s;
-        }
+    DF s = sh[(w < K ? w : 0) * kWarps + (lane & (kWarps - 1))];
+    for (int o = kWarps / 2; o > 0; o >>= 1)
+        s = df_add(s, DF{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
+    if (Sync::kCluster) {
+        if (w < K && lane < nb) store_remote(part + w * kClusterMax + blockIdx.x, s, lane);
+    } else {
+        if (w < K && lane == 0) part[w * nb + blockIdx.x] = s;
     }
 }
 
@@ -136,21 +139,28 @@ __device__ __forceinline__ void block_part(DF (&v)[K], DF *sh, DF *part, int nb)
 template <int K, class Sync>
 __device__ __forceinline__ void grid_total(const DF *part, int nb, DF *tot) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w < K) {
-        DF s{0.0f, 0.0f};
-        if (Sync::kCluster) {
-            if (lane < nb) s = part[w * kClusterMax + lane];
-        } else {
-            const float2 *p = reinterpret_cast<const float2 *>(part + w * nb);
-            for (int k = lane; k < nb; k += 32) {
-                const float2 v = __ldcg(p + k);
-                s = df_add(s, DF{v.x, v.y});
+    DF s{0.0f, 0.0f};
+    if (Sync::kCluster) {
+        const int b = lane & (kClusterMax - 1);
+        const DF v = part[(w < K ? w : 0) * kClusterMax + b];
+        s = DF{b < nb ? v.hi : 0.0f, b < nb ? v.lo : 0.0f};
+    } else {
+        const float2 *p = reinterpret_cast<const float2 *>(part + (w < K ? w : 0) * nb);
+        for (int k = 0; k < nb; k += 5 * 32) {
+            float2 v[5];
+#pragma unroll
+            for (int u = 0; u < 5; ++u) {
+                const int i = k + 32 * u + lane;
+                v[u] = make_float2(0.0f, 0.0f);
+                if (w < K && i < nb) v[u] = __ldcg(p + i);
             }
+#pragma unroll
+            for (int u = 0; u < 5; ++u) s = df_add(s, DF{v[u].x, v[u].y});
         }
-        for (int o = Sync::kCluster ? kClusterMax / 2 : 16; o > 0; o >>= 1)
-            s = df_add(s, DF{__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.lo, o)});
-        if (lane == 0) tot[w] = s;
     }
+    for (int o = Sync::kCluster ? kClusterMax / 2 : 16; o > 0; o >>= 1)
+        s = df_add(s, DF{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
+    if (w < K && lane == 0) tot[w] = s;
     __syncthreads();
 }
 
@@ -546,8 +556,6 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
     __shared__ double sh[2 * kPcgThreads + 16];   // FP64 sums; the double-float ones use its head
     __shared__ DF tot[3];
     __shared__ double scal[2];                    // FP64 scalars; 1: go on
-    __shared__ float coef;                        // alpha or beta
-    __shared__ int flag[2];                       // residual small: end the pass; replace in this cycle
     DF *shf = reinterpret_cast<DF *>(sh);
     const int nb = gridDim.x, n = a.n, L = M.nlev - 1;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -573,29 +581,33 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         for (int i = gtid; i < n; i += gstride) a.b[i] = a.b[i] - mean;
         Sync::sync();
     }
-    // solver scalars, kept by thread 0 in shared memory (no registers held
-    // across the loop by the other threads).  The step lengths are FP32 (x and
-    // r take the same alpha; any alpha near the minimiser keeps the recurrence
-    // consistent) and the recurrence's ||r||^2 double-float: a chain of FP64
-    // operations by one thread, a division among them, was 2 us of each of an
-    // iteration's two scalar steps.
-    __shared__ double t_tol2, t_rr, t_bb, t_rmax;
-    __shared__ DF t_rec;
-    __shared__ float t_rz;
-    __shared__ int t_it, t_status, t_updates, t_pass;
+    // Solver scalars, in shared memory (no registers held across the loop).
+    // The step lengths are FP32 (x and r take the same alpha; any alpha near
+    // the minimiser keeps the recurrence consistent) and the recurrence's
+    // ||r||^2 double-float, so every thread forms them from the totals itself:
+    // one thread's chain of FP64 operations, a division among them, was 2 us of
+    // each of an iteration's two scalar steps, its FP32 chain with a barrier
+    // after it 0.5 to 0.8.  FP32 values are compared with the largest FP32
+    // value not above an FP64 bound, which decides as the FP64 comparison.
+    // rz and rec: by the parity of the step, as some threads still read the
+    // last one's.
+    __shared__ double t_tol2, t_rr, t_bb;
+    __shared__ float t_small, t_fell;             // bounds of the recurrence's ||r||^2
+    __shared__ DF t_rec[2], t_rz[2];
+    __shared__ int t_status, t_updates, t_pass;
     if (threadIdx.x == 0) {
-        t_tol2 = t_rr = t_bb = t_rmax = 0.0;
-        t_rec = DF{0.0f, 0.0f};
-        t_rz = 0.0f;
-        t_it = 0; t_status = 1; t_updates = 0; t_pass = 0;
+        t_tol2 = t_rr = t_bb = 0.0;
+        t_status = 1; t_updates = 0; t_pass = 0;
     }
+    int it = 0;                                   // CG steps taken
+    float beta = 0.0f;
     // fresh: start a pass, from the FP64 true residual; else a CG step
-    bool fresh = true, first = true;
+    bool fresh = true;
     for (;;) {
         bool keep = false;
         if (fresh) {
             double bb = 0.0;
-            const double rr = true_residual(a, r, s0, om0, first, bb, gtid, gstride);
+            const double rr = true_residual(a, r, s0, om0, it == 0, bb, gtid, gstride);
             block_sum2(rr, bb, sh, ra, rb);
             if (threadIdx.x == 0) { partB[blockIdx.x] = ra; partD[blockIdx.x] = rb; }
             Sync::sync();
@@ -616,10 +628,11 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
                     ++t_updates;
                 }
                 ++t_pass;
-                t_rmax = t_rr;
-                t_rec = DF{(float)t_rr, 0.0f};
+                t_small = __double2float_rd(t_tol2);
+                t_fell = __double2float_rd(1e-6 * t_rr);
+                t_rec[it & 1] = DF{(float)t_rr, 0.0f};
                 if (t_rr <= t_tol2) { t_status = 0; scal[1] = 0.0; }
-                else if (t_it >= a.max_iter) { t_status = 1; scal[1] = 0.0; }
+                else if (it >= a.max_iter) { t_status = 1; scal[1] = 0.0; }
                 else if (stalled) { t_status = 3; scal[1] = 0.0; }
                 else scal[1] = 1.0;
             }
@@ -631,47 +644,39 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             // ||r - alpha Ap||^2 = ||r||^2 - 2 alpha r.Ap + alpha^2 Ap.Ap, which
             // only decides when the residual is replaced
             DF v[3];
-            const float beta = first ? 0.0f : coef;
-            if (M.lev[0].A.c16) direction_rows<true>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, first, v, gtid, gstride);
-            else direction_rows<false>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, first, v, gtid, gstride);
-            first = false;
+            if (M.lev[0].A.c16) direction_rows<true>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, gtid, gstride);
+            else direction_rows<false>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, gtid, gstride);
             CgUpdate up;
             up.load(a, gtid, gstride);
             block_part<3, Sync>(v, shf, partA, nb);
             Sync::sync();
             grid_total<3, Sync>(partA, nb, tot);
-            if (threadIdx.x == 0) {
-                ++t_it;
-                scal[1] = 1.0;
-                if (!(tot[0].hi > 0.0f)) { t_status = 2; scal[1] = 0.0; }
-                else {
-                    const float alpha = t_rz / tot[0].hi;
-                    coef = alpha;
-                    const DF rap{-2.0f * tot[1].hi, -2.0f * tot[1].lo};
-                    t_rec = df_add(t_rec, df_mul(df_add(df_mul(tot[2], alpha), rap), alpha));
-                    // replacement: at the end (tolerance or cap) by a new pass;
-                    // between (the recurrence fell by 1e6 in ||r||^2) inside
-                    // this cycle when L >= 2
-                    const double rec = (double)t_rec.hi;
-                    const bool small = rec <= t_tol2 || t_it >= a.max_iter, fell = rec <= 1e-6 * t_rmax;
-                    flag[0] = (small || (fell && L < 2)) ? 1 : 0;
-                    flag[1] = (!small && fell && L >= 2) ? 1 : 0;
-                }
+            const float pap = tot[0].hi;
+            DF rec = t_rec[it & 1];
+            const float alpha = t_rz[it & 1].hi / pap;
+            ++it;
+            if (!(pap > 0.0f)) {
+                if (threadIdx.x == 0) t_status = 2;
+                break;
             }
-            __syncthreads();
-            if (scal[1] == 0.0) break;
-            const float alpha = coef;
+            const DF rap{-2.0f * tot[1].hi, -2.0f * tot[1].lo};
+            rec = df_add(rec, df_mul(df_add(df_mul(tot[2], alpha), rap), alpha));
+            if (threadIdx.x == 0) t_rec[it & 1] = rec;
+            // replacement: at the end (tolerance or cap) by a new pass; between
+            // (the recurrence fell by 1e6 in ||r||^2) inside this cycle when
+            // L >= 2
+            const bool small = rec.hi <= t_small || it >= a.max_iter, fell = rec.hi <= t_fell;
             up.apply(a, s0, om0, alpha, gtid, gstride);
             for (int i = gtid + CgUpdate::R * gstride; i < n; i += CgUpdate::R * gstride) {
                 up.load(a, i, gstride);
                 up.apply(a, s0, om0, alpha, i, gstride);
             }
-            if (flag[0]) {
+            if (small || (fell && L < 2)) {
                 Sync::sync();
                 fresh = true;
                 continue;
             }
-            keep = flag[1] != 0;
+            keep = fell;
             // restriction of the new residual from that of the old one: one
             // gather per entry (of Ap) instead of two (r - alpha Ap), and r is
             // updated in place
@@ -742,26 +747,26 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         }
         block_part<1, Sync>(v, shf, partC, nb);
         Sync::sync();
-        grid_total<1, Sync>(partC, nb, tot);
-        if (keep) grid_sum2(partD, nullptr, nb, sh, ra, rb);
-        if (threadIdx.x == 0) {
-            scal[1] = 1.0;
-            if (keep) {
-                // the true residual replaces the recurrence's (as at a pass
-                // start, with the same stall test)
+        grid_total<1, Sync>(partC, nb, t_rz + (it & 1));
+        if (keep) {
+            // the true residual replaces the recurrence's (as at a pass start,
+            // with the same stall test)
+            grid_sum2(partD, nullptr, nb, sh, ra, rb);
+            if (threadIdx.x == 0) {
                 const bool stalled = ra > 1e-2 * t_rr;
-                t_rr = t_rmax = ra;
-                t_rec = DF{(float)ra, 0.0f};
+                t_rr = ra;
+                t_fell = __double2float_rd(1e-6 * t_rr);
+                t_rec[it & 1] = DF{(float)ra, 0.0f};
                 ++t_updates;
+                scal[1] = 1.0;
                 if (t_rr <= t_tol2) { t_status = 0; scal[1] = 0.0; }
                 else if (stalled) { t_status = 3; scal[1] = 0.0; }
             }
-            // the direction continues across replacements
-            coef = first ? 0.0f : tot[0].hi / t_rz;
-            t_rz = tot[0].hi;
+            __syncthreads();
+            if (scal[1] == 0.0) break;
         }
-        __syncthreads();
-        if (scal[1] == 0.0) break;
+        // the direction continues across replacements
+        beta = it == 0 ? 0.0f : t_rz[it & 1].hi / t_rz[(it & 1) ^ 1].hi;
         fresh = false;
     }
     if (a.remove_mean) {
@@ -778,7 +783,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         for (int i = gtid; i < n; i += gstride) a.x[i] = a.x[i] - mean;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *a.out_iter = t_it;
+        *a.out_iter = it;
         *a.out_status = t_status;
         *a.out_rr = t_rr;
         *a.out_bb = t_bb;
