@@ -36,6 +36,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "pg_device.cuh"
@@ -164,6 +165,29 @@ __device__ __forceinline__ void grid_total(const DF *part, int nb, DF *tot) {
     __syncthreads();
 }
 
+// ---- the work of a block ------------------------------------------------------
+// The threads of nb blocks, b this block's number among them.  Row r (or, with
+// g lanes a row, lane r g + k) of a product goes to the r-th of them, in one of
+// two orders: block by block, or (spread) the first warp of every block, then
+// the second ones.  Spread where the level-0 rows are at most one per thread: its
+// coarse products then have fewer rows than threads, and block by block
+// the first blocks worked and the others waited (39k rows: a product over
+// 4,136 rows in 16 of 77 blocks).  Block by block above, where a block's rows
+// should be neighbours that share gathered lines.  Solve, block by block ->
+// spread: 4,096 rows 0.30 -> 0.26 ms, 21,952 0.61 -> 0.56, 39,298 0.54 -> 0.51,
+// 68,908 0.59 -> 0.57; 13,824 (16 blocks) 0.475 -> 0.50.
+// (Equal contiguous ranges per block, which leave no block a round of rows more
+// than another, measured 1 to 5% slower than either at all sizes.)
+struct Span {
+    int b, nb;
+    bool spread;
+    __device__ __forceinline__ int first() const {
+        const int w = threadIdx.x >> 5;
+        return 32 * (spread ? w * nb + b : b * kWarps + w) + (int)(threadIdx.x & 31);
+    }
+    __device__ __forceinline__ int stride() const { return kPcgThreads * nb; }
+};
+
 // ---- products ---------------------------------------------------------------
 // Read-only loads of operator entries that ask the L2 for the 256-byte
 // segment around the address, so a row's next chunks arrive with this one.
@@ -286,8 +310,8 @@ __device__ __forceinline__ float a0_sum(const SpOp &A, const float *x, int off, 
 struct SellHead {
     int2 h = {0, 0};
     int end = 0;
-    __device__ __forceinline__ void load(const SpOp &S, int r) {
-        if (r < S.n) {
+    __device__ __forceinline__ void load(const SpOp &S, int r, int r1) {
+        if (r < r1) {
             h = __ldg(S.head + (r >> 5));
             end = __ldg(&S.head[(r >> 5) + 1].x);
         }
@@ -296,24 +320,26 @@ struct SellHead {
     __device__ __forceinline__ int width() const { return (end - h.x) >> 5; }
 };
 
-// e.row(i, (S x)_i, e.pre(i)) for every row i, over the threads t0, t0 + ts,
-// ...  pre loads the row's other operands before its gathers start.  A phase
-// is a chain of dependent trips per thread (head -> entries -> gathers) over
-// 32 warps of an SM; what an earlier form kept in flight per thread beyond a
-// row (two and four rows together, 128 registers) cost more in code and
-// warps than it hid (100^3 solve 4.12 ms against 3.38).
+// e.row(i, (S x)_i, e.pre(i)) for every row i, over the blocks of sp.  pre
+// loads the row's other operands before its gathers start.  A phase is a chain
+// of dependent trips per thread (head -> entries -> gathers) over 32 warps of an
+// SM; what an earlier form kept in flight per thread beyond a row (two and
+// four rows together, 128 registers) cost more in code and warps than it hid
+// (100^3 solve 4.12 ms against 3.38).
 // CSR: g <= 32 lanes a row, two chunks per lane and step, reduced by shuffles
 // (all lanes run the same rounds); g = 64..512: the warps of one block a row,
-// reduced through shared memory ((t0, ts) cover whole blocks).
+// reduced through shared memory.
 template <class F, class E>
-__device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, int t0, int ts) {
+__device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, Span sp) {
     const int g = S.g;
     if (g == 1) {
+        int i = sp.first();
+        const int i1 = S.n, st = sp.stride();
         SellHead h;
-        h.load(S, t0);
-        for (int i = t0; i < S.n; i += ts) {
+        h.load(S, i, i1);
+        for (; i < i1; i += st) {
             const int off = h.off(i), w = h.width(), cb = h.h.y;
-            h.load(S, i + ts);
+            h.load(S, i + st, i1);
             const typename E::Pre pv = e.pre(i);
             e.row(i, sell_sum<F, 3>(S, x, off, w, cb), pv);
         }
@@ -321,20 +347,20 @@ __device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, i
     }
     const bool wide = g > 32;
     __shared__ float red[kWarps];
-    const int lane = wide ? threadIdx.x & (g - 1) : t0 & (g - 1);
-    const int per_block = blockDim.x / g;
-    const int grp = wide ? (t0 / (int)blockDim.x) * per_block + threadIdx.x / g : t0 / g;
-    const int ngrp = wide ? (ts / (int)blockDim.x) * per_block : ts / g;
-    const int rounds = (S.n + ngrp - 1) / ngrp;
+    const int sh = 31 - __clz(g), lane = threadIdx.x & (g - 1);
+    const int pb = kPcgThreads >> sh;              // rows per block and round
+    const int i1 = S.n, step = pb * sp.nb;
+    int i = wide ? sp.b * pb + (int)(threadIdx.x >> sh) : sp.first() >> sh;
+    const int rounds = (S.n + step - 1) / step;
     int2 h = make_int2(0, 0);
     int end = 0;
-    if (grp < S.n) { h = __ldg(S.head + grp); end = __ldg(&S.head[grp + 1].x); }
-    for (int t = 0; t < rounds; ++t) {
-        const int i = grp + t * ngrp, in = i + ngrp;
-        const int off = h.x, cb = h.y, len = i < S.n ? end - h.x : 0;
-        if (in < S.n) { h = __ldg(S.head + in); end = __ldg(&S.head[in + 1].x); }
+    if (i < i1) { h = __ldg(S.head + i); end = __ldg(&S.head[i + 1].x); }
+    for (int t = 0; t < rounds; ++t, i += step) {
+        const int in = i + step;
+        const int off = h.x, cb = h.y, len = i < i1 ? end - h.x : 0;
+        if (in < i1) { h = __ldg(S.head + in); end = __ldg(&S.head[in + 1].x); }
         typename E::Pre pv{};
-        if (i < S.n && lane == 0) pv = e.pre(i);
+        if (i < i1 && lane == 0) pv = e.pre(i);
         float sum = 0.0f;
         for (int k = lane; k < len; k += 2 * g) {
             F f[2];
@@ -361,7 +387,7 @@ __device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, i
             }
             __syncthreads();
         }
-        if (lane == 0 && i < S.n) e.row(i, F::kHalf ? sum * S.vscale : sum, pv);
+        if (lane == 0 && i < i1) e.row(i, F::kHalf ? sum * S.vscale : sum, pv);
     }
 }
 
@@ -370,10 +396,10 @@ __device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, i
 // unless a slice or row spans more; the others (G, the coarsest inverse) FP32
 // and 32-bit columns.
 template <bool V16, class E>
-__device__ __forceinline__ void product(const SpOp &S, const float *x, E &e, int t0, int ts) {
-    if (V16 && S.c16) product_f<FmtH16>(S, x, e, t0, ts);
-    else if (V16) product_f<FmtH32>(S, x, e, t0, ts);
-    else product_f<FmtF32>(S, x, e, t0, ts);
+__device__ __forceinline__ void product(const SpOp &S, const float *x, E &e, Span sp) {
+    if (V16 && S.c16) product_f<FmtH16>(S, x, e, sp);
+    else if (V16) product_f<FmtH32>(S, x, e, sp);
+    else product_f<FmtF32>(S, x, e, sp);
 }
 
 // ---- what a product's rows become -------------------------------------------
@@ -428,15 +454,15 @@ struct DirectRow {
 // diagonal is not read.
 template <bool C16, class F>
 __device__ __forceinline__ DF prolong_rows(const SpOp &A, const SpOp &S, const float *s, const float *y, const float *r,
-                                           const float *dinv, float om, float *z, int t0, int ts) {
+                                           const float *dinv, float om, float *z, int i0, int i1, int gst) {
     DF rz{0.0f, 0.0f};
     SellHead ha, hs;
-    ha.load(A, t0);
-    hs.load(S, t0);
-    for (int i = t0; i < A.n; i += ts) {
+    ha.load(A, i0, i1);
+    hs.load(S, i0, i1);
+    for (int i = i0; i < i1; i += gst) {
         const int oa = ha.off(i), wa = ha.width(), ca = ha.h.y, os = hs.off(i), ws = hs.width(), cs = hs.h.y;
-        ha.load(A, i + ts);
-        hs.load(S, i + ts);
+        ha.load(A, i + gst, i1);
+        hs.load(S, i + gst, i1);
         const float si = s[i], ri = r[i], di = __ldg(dinv + i);
         const float q = a0_sum<C16>(A, s, oa, wa, ca);
         const float u = sell_sum<F, 3>(S, y, os, ws, cs);
@@ -451,13 +477,13 @@ __device__ __forceinline__ DF prolong_rows(const SpOp &A, const SpOp &S, const f
 // first step), and this thread's shares of p.Ap, r.Ap and Ap.Ap.
 template <bool C16>
 __device__ __forceinline__ void direction_rows(const SpOp &A, const float *diag, const float *z, const float *r,
-                                               float *p, float *Ap, float beta, bool first, DF (&v)[3], int t0, int ts) {
+                                               float *p, float *Ap, float beta, bool first, DF (&v)[3], int i0, int i1, int gst) {
     float pap = 0.0f, rap = 0.0f, apap = 0.0f;
     SellHead h;
-    h.load(A, t0);
-    for (int i = t0; i < A.n; i += ts) {
+    h.load(A, i0, i1);
+    for (int i = i0; i < i1; i += gst) {
         const int off = h.off(i), w = h.width(), cb = h.h.y;
-        h.load(A, i + ts);
+        h.load(A, i + gst, i1);
         const float zi = z[i], ri = r[i], di = __ldg(diag + i);
         const float p0 = first ? 0.0f : p[i], q0 = first ? 0.0f : Ap[i];
         const float s = fmaf(di, zi, a0_sum<C16>(A, z, off, w, cb));
@@ -487,9 +513,9 @@ __device__ __forceinline__ int split_point(const SpOp &A, const SpOp &B, int nb)
 // FP32 and, with s, omega D^-1 r into s; returns this thread's share of
 // ||b - A x||^2 and, with want_bb, adds its share of ||b||^2 to bb.
 __device__ __forceinline__ double true_residual(const PcgArgs &a, float *r, float *s, float om, bool want_bb, double &bb,
-                                             int t0, int ts) {
+                                             int i0, int i1, int gst) {
     double rr = 0.0;
-    for (int i = t0; i < a.n; i += ts) {
+    for (int i = i0; i < i1; i += gst) {
         double q = 0.0;
         const int64_t base = a.slice_ptr[i >> 5] + (i & 31);
         const int w = a.slice_width[i >> 5];
@@ -508,9 +534,9 @@ __device__ __forceinline__ double true_residual(const PcgArgs &a, float *r, floa
 
 // The level-0 restriction, at three places of the loop: one copy.
 __device__ __noinline__ void restrict0(const SpOp &S, const float *x, float *b, float *sb, const float *dinv, float om,
-                                       float alpha, bool update, int t0, int ts) {
+                                       float alpha, bool update, Span sp) {
     RestrictRow e{b, sb, dinv, om, alpha, update};
-    product<true>(S, x, e, t0, ts);
+    product<true>(S, x, e, sp);
 }
 
 // x += alpha p, r -= alpha Ap, s = omega D^-1 r of this thread's rows.  The
@@ -520,11 +546,11 @@ struct CgUpdate {
     static constexpr int R = 4;
     double x[R];
     float p[R], q[R], r[R], d[R];
-    __device__ __forceinline__ void load(const PcgArgs &a, int i, int ts) {
+    __device__ __forceinline__ void load(const PcgArgs &a, int i, int i1, int gst) {
 #pragma unroll
         for (int k = 0; k < R; ++k) {
-            const int j = i + k * ts;
-            const bool ok = j < a.n;
+            const int j = i + k * gst;
+            const bool ok = j < i1;
             x[k] = ok ? a.x[j] : 0.0;
             p[k] = ok ? a.p32[j] : 0.0f;
             q[k] = ok ? a.Ap32[j] : 0.0f;
@@ -532,11 +558,11 @@ struct CgUpdate {
             d[k] = ok ? __ldg(a.dinv32 + j) : 0.0f;
         }
     }
-    __device__ __forceinline__ void apply(const PcgArgs &a, float *s, float om, float alpha, int i, int ts) const {
+    __device__ __forceinline__ void apply(const PcgArgs &a, float *s, float om, float alpha, int i, int i1, int gst) const {
 #pragma unroll
         for (int k = 0; k < R; ++k) {
-            const int j = i + k * ts;
-            if (j < a.n) {
+            const int j = i + k * gst;
+            if (j < i1) {
                 const float n = fmaf(-alpha, q[k], r[k]);
                 a.x[j] = fma((double)alpha, (double)p[k], x[k]);
                 a.r32[j] = n;
@@ -558,8 +584,8 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
     __shared__ double scal[2];                    // FP64 scalars; 1: go on
     DF *shf = reinterpret_cast<DF *>(sh);
     const int nb = gridDim.x, n = a.n, L = M.nlev - 1;
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gstride = nb * blockDim.x;
+    const Span all{(int)blockIdx.x, nb, n <= nb * kPcgThreads};
+    const int i0 = all.first(), i1 = n, gst = all.stride();
     __shared__ DF part_cluster[Sync::kCluster ? 4 * kClusterMax : 1];
     DF *partA = Sync::kCluster ? part_cluster : reinterpret_cast<DF *>(a.partials);
     DF *partC = partA + 3 * (Sync::kCluster ? kClusterMax : nb);
@@ -570,7 +596,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
 
     if (a.remove_mean) {
         double s = 0.0;
-        for (int i = gtid; i < n; i += gstride) s += a.b[i];
+        for (int i = i0; i < i1; i += gst) s += a.b[i];
         block_sum2(s, 0.0, sh, ra, rb);
         if (threadIdx.x == 0) partD[blockIdx.x] = ra;
         Sync::sync();
@@ -578,7 +604,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         if (threadIdx.x == 0) scal[0] = ra / (double)n;
         __syncthreads();
         const double mean = scal[0];
-        for (int i = gtid; i < n; i += gstride) a.b[i] = a.b[i] - mean;
+        for (int i = i0; i < i1; i += gst) a.b[i] = a.b[i] - mean;
         Sync::sync();
     }
     // Solver scalars, in shared memory (no registers held across the loop).
@@ -607,7 +633,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         bool keep = false;
         if (fresh) {
             double bb = 0.0;
-            const double rr = true_residual(a, r, s0, om0, it == 0, bb, gtid, gstride);
+            const double rr = true_residual(a, r, s0, om0, it == 0, bb, i0, i1, gst);
             block_sum2(rr, bb, sh, ra, rb);
             if (threadIdx.x == 0) { partB[blockIdx.x] = ra; partD[blockIdx.x] = rb; }
             Sync::sync();
@@ -638,16 +664,16 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             }
             __syncthreads();
             if (scal[1] == 0.0) break;
-            if (L >= 2) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, gtid, gstride);
+            if (L >= 2) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
         } else {
             // p = z + beta p, Ap = A z + beta Ap; p.Ap and the terms of
             // ||r - alpha Ap||^2 = ||r||^2 - 2 alpha r.Ap + alpha^2 Ap.Ap, which
             // only decides when the residual is replaced
             DF v[3];
-            if (M.lev[0].A.c16) direction_rows<true>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, gtid, gstride);
-            else direction_rows<false>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, gtid, gstride);
+            if (M.lev[0].A.c16) direction_rows<true>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
+            else direction_rows<false>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
             CgUpdate up;
-            up.load(a, gtid, gstride);
+            up.load(a, i0, i1, gst);
             block_part<3, Sync>(v, shf, partA, nb);
             Sync::sync();
             grid_total<3, Sync>(partA, nb, tot);
@@ -666,10 +692,10 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             // (the recurrence fell by 1e6 in ||r||^2) inside this cycle when
             // L >= 2
             const bool small = rec.hi <= t_small || it >= a.max_iter, fell = rec.hi <= t_fell;
-            up.apply(a, s0, om0, alpha, gtid, gstride);
-            for (int i = gtid + CgUpdate::R * gstride; i < n; i += CgUpdate::R * gstride) {
-                up.load(a, i, gstride);
-                up.apply(a, s0, om0, alpha, i, gstride);
+            up.apply(a, s0, om0, alpha, i0, i1, gst);
+            for (int i = i0 + CgUpdate::R * gst; i < i1; i += CgUpdate::R * gst) {
+                up.load(a, i, i1, gst);
+                up.apply(a, s0, om0, alpha, i, i1, gst);
             }
             if (small || (fell && L < 2)) {
                 Sync::sync();
@@ -680,43 +706,43 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             // restriction of the new residual from that of the old one: one
             // gather per entry (of Ap) instead of two (r - alpha Ap), and r is
             // updated in place
-            if (L >= 2) restrict0(M.lev[0].ST, a.Ap32, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, alpha, true, gtid, gstride);
+            if (L >= 2) restrict0(M.lev[0].ST, a.Ap32, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, alpha, true, all);
         }
         Sync::sync();
         // z = B r
         const float *yup = M.yL;
         if (L == 1) {
             RestrictRow e{M.yL, nullptr, nullptr, 0.0f, 0.0f, false};
-            product<false>(M.G, r, e, gtid, gstride);
+            product<false>(M.G, r, e, all);
             Sync::sync();
         }
         for (int l = 1; l < L; ++l) {
             // the restriction to the next level (or G) and the smoothing W_l
             const bool coarse = l == L - 1;
             const AmgLevelDev &V = M.lev[l];
-            int my = -1, pt0 = gtid, pts = gstride;
+            int my = -1;
+            Span sp = all;
             if (nb > 1) {
                 const int cut = coarse ? split_point(M.G, V.A, nb) : split_point(V.ST, V.A, nb);
                 my = (int)blockIdx.x < cut ? 0 : 1;
-                pt0 = gtid - my * cut * (int)blockDim.x;
-                pts = (my ? nb - cut : cut) * (int)blockDim.x;
+                sp = my ? Span{(int)blockIdx.x - cut, nb - cut, all.spread} : Span{(int)blockIdx.x, cut, all.spread};
             }
             if (my != 1) {
                 const AmgLevelDev &N = M.lev[coarse ? l : l + 1];
                 RestrictRow e{coarse ? M.yL : N.b, coarse ? nullptr : N.sb, N.dinv, N.omega, 0.0f, false};
-                if (coarse) product<false>(M.G, V.b, e, pt0, pts);
-                else product<true>(V.ST, V.b, e, pt0, pts);
+                if (coarse) product<false>(M.G, V.b, e, sp);
+                else product<true>(V.ST, V.b, e, sp);
             }
             if (my != 0) {
                 SmoothRow w{V.t, V.sb, V.dinv, V.omega};
-                product<true>(V.A, V.sb, w, pt0, pts);
+                product<true>(V.A, V.sb, w, sp);
             }
             if (keep && coarse) {
                 // replacement inside the cycle: the FP64 true residual of x
                 // (complete here) into r; z = B r of the recurrence's r stands
                 // for B of the true one (they differ by the recurrence's drift)
                 double unused = 0.0;
-                const double rr = true_residual(a, r, nullptr, 0.0f, false, unused, gtid, gstride);
+                const double rr = true_residual(a, r, nullptr, 0.0f, false, unused, i0, i1, gst);
                 block_sum2(rr, 0.0, sh, ra, rb);
                 if (threadIdx.x == 0) partD[blockIdx.x] = ra;
             }
@@ -724,8 +750,8 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         }
         if (L >= 2) {
             AddRow e{M.y1, M.lev[1].t};
-            product<true>(M.U1, M.stack, e, gtid, gstride);
-            if (keep) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, gtid, gstride);
+            product<true>(M.U1, M.stack, e, all);
+            if (keep) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
             Sync::sync();
             yup = M.y1;
         }
@@ -733,16 +759,16 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         if (L >= 1) {
             const SpOp &A0 = M.lev[0].A;
             if (A0.c16 && M.S0.c16)
-                v[0] = prolong_rows<true, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, gtid, gstride);
+                v[0] = prolong_rows<true, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
             else if (M.S0.c16)
-                v[0] = prolong_rows<false, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, gtid, gstride);
+                v[0] = prolong_rows<false, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
             else if (A0.c16)
-                v[0] = prolong_rows<true, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, gtid, gstride);
+                v[0] = prolong_rows<true, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
             else
-                v[0] = prolong_rows<false, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, gtid, gstride);
+                v[0] = prolong_rows<false, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
         } else {
             DirectRow e{z, r, DF{0.0f, 0.0f}};
-            product<false>(M.cinv, r, e, gtid, gstride);
+            product<false>(M.cinv, r, e, all);
             v[0] = e.rz;
         }
         block_part<1, Sync>(v, shf, partC, nb);
@@ -772,7 +798,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
     if (a.remove_mean) {
         Sync::sync();
         double s = 0.0;
-        for (int i = gtid; i < n; i += gstride) s += a.x[i];
+        for (int i = i0; i < i1; i += gst) s += a.x[i];
         block_sum2(s, 0.0, sh, ra, rb);
         if (threadIdx.x == 0) partB[blockIdx.x] = ra;
         Sync::sync();
@@ -780,7 +806,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
         if (threadIdx.x == 0) scal[0] = ra / (double)n;
         __syncthreads();
         const double mean = scal[0];
-        for (int i = gtid; i < n; i += gstride) a.x[i] = a.x[i] - mean;
+        for (int i = i0; i < i1; i += gst) a.x[i] = a.x[i] - mean;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.out_iter = it;
@@ -798,10 +824,11 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
 // barrier is the hardware's (0.3 against 1.3 us of a cooperative grid, five
 // times an iteration) and its sums stay in shared memory, while its 16 SMs are
 // enough for so few rows.  Measured, solve on the grid -> on the cluster: 2,744
-// rows 0.84 -> 0.51 ms, 9,260 0.55 -> 0.42, 13,824 0.57 -> 0.51; 21,952 0.69 -> 0.74
-// and 39,298 0.61 -> 0.93, so the line lies between.  Rows per block: 1,000 rows
-// 0.50 / 0.38 / 0.33 / 0.29 ms with 512 / 256 / 128 / 64.
-constexpr int kClusterRows = 16384, kClusterRowsPerBlock = 64;
+// rows 0.84 -> 0.45 ms, 9,260 0.49 -> 0.385, 13,824 0.467 -> 0.474 and, periodic, 0.64
+// -> 0.66, 39,298 0.61 -> 0.93, so the line lies between the second and the
+// third.  Rows per block: 1,000 rows 0.50 / 0.38 / 0.33 / 0.29 ms with 512 / 256 /
+// 128 / 64.
+constexpr int kClusterRows = 12288, kClusterRowsPerBlock = 64;
 
 int pcg_amg_grid_blocks() {
     static int g = 0;
@@ -862,8 +889,12 @@ int launch_pcg_amg(const PcgArgs &a, const AmgDev &amg, cudaStream_t st) {
         return (int)cudaLaunchKernelExC(&cfg, (const void *)k_pcg_amg<ClusterSync>, params);
     }
     int nb = pcg_amg_grid_blocks();
-    const int need = (a.n + kPcgThreads - 1) / kPcgThreads;
-    if (need < nb) nb = need < 1 ? 1 : need;
+    // one row per thread where the blocks suffice; below one block per SM twice
+    // as many, so that the coarse products have the idle SMs (39,298 rows: 0.51 ms
+    // with 77 blocks, 0.48 with 152; four times as many lose to the barrier: 21,952
+    // rows 0.56 ms with 43, 0.55 with 86, 0.60 with 152)
+    const int need = (a.n + kPcgThreads - 1) / kPcgThreads, sms = sm_count();
+    if (need < nb) nb = need > sms ? need : std::max(need, std::min(sms, 2 * need));
     return (int)cudaLaunchCooperativeKernel((const void *)k_pcg_amg<GridSync>, dim3(nb), dim3(kPcgThreads), params, 0, st);
 }
 

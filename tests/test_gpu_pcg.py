@@ -1,6 +1,6 @@
 """The AMG-PCG solve against a direct solve on hierarchies of one level (the
 dense inverse), two and three, operators in natural and random order, systems
-of one block, of a cluster (up to 16,384 rows) and of a grid, row counts that are
+of one block, of a cluster (up to 12,288 rows) and of a grid, row counts that are
 no multiple of a slice."""
 import numpy as np
 import pytest
@@ -50,6 +50,34 @@ def test_probe_solve(lib, n, order):
     want = np.where(kind == 1, -1.5, 0.0)
     b = (M @ rho - K @ want)[free]
     want[free] = spl.spsolve(K[free][:, free].tocsc(), b)
+    assert np.abs(phi - want).max() <= 1e-9 * np.abs(want).max()
+    assert solver.last_info.residual <= 1e-12 * solver.last_info.rhs_norm * 1.0001
+    again = solver.solve(punc.Function(pop, "phi"), None, [punc.Object(2, potential=-1.5)])
+    assert np.array_equal(again, phi)
+    pop.close()
+
+
+@pytest.mark.parametrize("n", [24, 34, 42, 54])
+def test_grid_solve(lib, n):
+    """The grid's forms: two blocks per 512 rows (15k rows), one block per SM
+    (42k), one per 512 rows (79k), more rows than threads (166k), against
+    a CG of the host at a residual of 1e-13, with the bound of test_probe_solve."""
+    rng = np.random.default_rng(n)
+    ma = meshgen.probe_box(n, 2.0, 0.9)
+    mesh = punc.Mesh(ma)
+    K, M = matrices(mesh)
+    kind = mesh.table(L.T_BC_KIND)
+    pop = punc.Population(mesh, warm_start=0)
+    rho = rng.normal(size=mesh.n_dofs)
+    punc.Function(pop, "rho").set_local(rho)
+    solver = punc.PoissonSolver(pop)
+    phi = solver.solve(punc.Function(pop, "phi"), None, [punc.Object(2, potential=-1.5)])
+    free = np.nonzero(kind < 0)[0]
+    want = np.where(kind == 1, -1.5, 0.0)
+    b = (M @ rho - K @ want)[free]
+    A = K[free][:, free]
+    want[free], status = spl.cg(A, b, rtol=1e-13, atol=0.0, maxiter=5000, M=sp.diags(1.0 / A.diagonal()))
+    assert status == 0
     assert np.abs(phi - want).max() <= 1e-9 * np.abs(want).max()
     assert solver.last_info.residual <= 1e-12 * solver.last_info.rhs_norm * 1.0001
     again = solver.solve(punc.Function(pop, "phi"), None, [punc.Object(2, potential=-1.5)])
