@@ -20,10 +20,12 @@
 // Arithmetic in T (double for the FP64 form, float for the mixed form); the
 // residual's norm in FP64.
 //
-// What bounds it: the chain of loads of a row (entries, then gathers) and the
-// barrier of each iteration; in FP64 also the 45 FP64 operations of a row at
-// 1/64 of the FP32 rate.  Measured against the CG form (GB300, solve with rhs
-// and packing): FP64 9,260 dofs 563 -> 265 us, FP32 39,298 dofs 372 -> 106 us.
+// What bounds it: the gathers and the barrier of each iteration; in FP64 also
+// the 45 FP64 operations of a row at 1/64 of the FP32 rate; in the form for
+// larger systems (k_mass_cheb3), which reads the matrix each time, the chain of
+// loads of a row.  Measured (GB300, solve with rhs and packing), CG -> that form ->
+// rows in registers (k_mass_cheb3_reg): FP64 9,260 dofs 563 -> 266 -> 101 us, FP32
+// 39,298 dofs 372 -> 117 -> 75 us.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -142,9 +144,9 @@ __device__ __forceinline__ V3<T> mass_row(const Cheb3Args<T> &a, const T *v, int
         for (int q = 0; q < C; ++q) g[q] = load3(v, c[q]);
 #pragma unroll
         for (int q = 0; q < C; ++q) {
-            s.x += m[q] * g[q].x;
-            s.y += m[q] * g[q].y;
-            s.z += m[q] * g[q].z;
+            s.x = fma(m[q], g[q].x, s.x);
+            s.y = fma(m[q], g[q].y, s.y);
+            s.z = fma(m[q], g[q].z, s.z);
         }
     }
     return s;
@@ -156,12 +158,78 @@ __device__ __forceinline__ int iterations_left(double rr, double tol2, float sla
     return max(1, min(64, (int)ceilf((slack + 0.5f * logf(ratio2)) / kRate)));
 }
 
+// What the blocks decide together, each for itself from the same sums.
+struct Checks {
+    double tol2[3], rr[3], bb[3];
+    int next_check, done, cold[3];
+};
+
+// The first residual and right-hand side (loc: this thread's squares, three
+// components each) against the tolerance: the iterations needed, and the
+// components whose start is worse than zero and is dropped.  One grid barrier.
+template <typename T>
+__device__ void first_check(const Cheb3Args<T> &a, const double (&loc)[6], int nb, double *sh, Checks &S) {
+    double out[6];
+    block_sum_n<6>(loc, sh, out);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 6; ++k) a.partials[k * nb + blockIdx.x] = out[k];
+    cg::this_grid().sync();
+    grid_sum_n<6>(a.partials, nb, out);
+    if (threadIdx.x < 32) {
+        // one lane per component
+        const int c = threadIdx.x;
+        int need = 0;
+        double v = 0.0, u = 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double r0 = __shfl_sync(0xffffffffu, out[q], 0), b0 = __shfl_sync(0xffffffffu, out[3 + q], 0);
+            if (c == q) { v = r0; u = b0; }
+        }
+        if (c < 3) {
+            const double tol = fmax(a.rtol * sqrt(u), a.atol);
+            S.cold[c] = v > u;
+            v = fmin(v, u);
+            S.rr[c] = v;
+            S.bb[c] = u;
+            S.tol2[c] = tol * tol;
+            // 1 / T_k(theta / delta) = 2 exp(-rate k) <= tol / ||r||, and three
+            // iterations more: the error of the slowest modes, which CG
+            // damps below its residual, is then below CG's too (16^3 to
+            // 31^3, CG1 runs: phi within 2e-11 of a 64-bit run, CG 1.1e-10)
+            if (v > tol * tol) need = iterations_left(v, tol * tol, 3.5f);
+        }
+        need = max(need, __shfl_down_sync(0xffffffffu, need, 2));
+        need = max(need, __shfl_down_sync(0xffffffffu, need, 1));
+        if (c == 0) {
+            S.next_check = min(need, a.max_iter);
+            S.done = need == 0;
+        }
+    }
+    __syncthreads();
+}
+
+// A later residual (part: the blocks' sums, complete): met, or more iterations.
+template <typename T>
+__device__ void later_check(const Cheb3Args<T> &a, const double *part, int nb, int it, Checks &S) {
+    double out[3];
+    grid_sum_n<3>(part, nb, out);
+    if (threadIdx.x == 0) {
+        int need = 0;
+        for (int c = 0; c < 3; ++c) {
+            S.rr[c] = out[c];
+            if (S.rr[c] > S.tol2[c]) need = max(need, iterations_left(S.rr[c], S.tol2[c], 0.0f));
+        }
+        S.done = need == 0;
+        S.next_check = min(it + need, a.max_iter);
+    }
+    __syncthreads();
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ Cheb3Args<T> a) {
     cg::grid_group grid = cg::this_grid();
     __shared__ double sh[16 * 6];
-    __shared__ double tol2[3], rr[3], bb[3];
-    __shared__ int next_check, done, cold[3];
+    __shared__ Checks S;
     const int nb = gridDim.x, n = a.n;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gs = nb * blockDim.x;
     T *d = a.d0, *dn = a.d1;
@@ -194,52 +262,15 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
             loc[4] += (double)b.y * (double)b.y;
             loc[5] += (double)b.z * (double)b.z;
         }
-        double out[6];
-        block_sum_n<6>(loc, sh, out);
-        if (threadIdx.x == 0)
-            for (int k = 0; k < 6; ++k) a.partials[k * nb + blockIdx.x] = out[k];
-        grid.sync();
-        grid_sum_n<6>(a.partials, nb, out);
-        if (threadIdx.x < 32) {
-            // one lane per component
-            const int c = threadIdx.x;
-            int need = 0;
-            double v = 0.0, u = 0.0;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const double r0 = __shfl_sync(0xffffffffu, out[q], 0), b0 = __shfl_sync(0xffffffffu, out[3 + q], 0);
-                if (c == q) { v = r0; u = b0; }
-            }
-            if (c < 3) {
-                const double tol = fmax(a.rtol * sqrt(u), a.atol);
-                // a start that is worse than zero is dropped
-                cold[c] = v > u;
-                v = fmin(v, u);
-                rr[c] = v;
-                bb[c] = u;
-                tol2[c] = tol * tol;
-                // 1 / T_k(theta / delta) = 2 exp(-rate k) <= tol / ||r||, and three
-                // iterations more: the error of the slowest modes, which CG
-                // damps below its residual, is then below CG's too (16^3 to
-                // 31^3, CG1 runs: phi within 2e-11 of a 64-bit run, CG 1.1e-10)
-                if (v > tol * tol) need = iterations_left(v, tol * tol, 3.5f);
-            }
-            need = max(need, __shfl_down_sync(0xffffffffu, need, 2));
-            need = max(need, __shfl_down_sync(0xffffffffu, need, 1));
-            if (c == 0) {
-                next_check = min(need, a.max_iter);
-                done = need == 0;
-            }
-        }
-        __syncthreads();
-        if (cold[0] || cold[1] || cold[2]) {
+        first_check(a, loc, nb, sh, S);
+        if (S.cold[0] || S.cold[1] || S.cold[2]) {
             for (int i = gtid; i < n; i += gs) {
                 const V3<T> b = load3(dn, i);
                 V3<T> x = load3(a.x, i), r = load3(a.r, i), di = load3(d, i);
                 const T f = a.dinv[i] * (T)(1.0 / kTheta);
-                if (cold[0]) { x.x = 0; r.x = b.x; di.x = f * b.x; }
-                if (cold[1]) { x.y = 0; r.y = b.y; di.y = f * b.y; }
-                if (cold[2]) { x.z = 0; r.z = b.z; di.z = f * b.z; }
+                if (S.cold[0]) { x.x = 0; r.x = b.x; di.x = f * b.x; }
+                if (S.cold[1]) { x.y = 0; r.y = b.y; di.y = f * b.y; }
+                if (S.cold[2]) { x.z = 0; r.z = b.z; di.z = f * b.z; }
                 store3(a.x, i, x);
                 store3(a.r, i, r);
                 store3(d, i, di);
@@ -248,9 +279,9 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
         }
     }
     int it = 0;
-    while (!done && it < a.max_iter) {
+    while (!S.done && it < a.max_iter) {
         ++it;
-        const bool check = it == next_check;
+        const bool check = it == S.next_check;
         const T c1 = a.c1[min(it, kCheb) - 1], c2 = a.c2[min(it, kCheb) - 1];
         double *part = a.partials + (size_t)(6 + 3 * (it & 1)) * nb;   // read by all before it is written again
         double loc[3] = {0, 0, 0};
@@ -272,26 +303,14 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
         T *t = d;
         d = dn;
         dn = t;
-        double out[3];
         if (check) {
+            double out[3];
             block_sum_n<3>(loc, sh, out);
             if (threadIdx.x == 0)
                 for (int k = 0; k < 3; ++k) part[k * nb + blockIdx.x] = out[k];
         }
         grid.sync();
-        if (check) {
-            grid_sum_n<3>(part, nb, out);
-            if (threadIdx.x == 0) {
-                int need = 0;
-                for (int c = 0; c < 3; ++c) {
-                    rr[c] = out[c];
-                    if (rr[c] > tol2[c]) need = max(need, iterations_left(rr[c], tol2[c], 0.0f));
-                }
-                done = need == 0;
-                next_check = min(it + need, a.max_iter);
-            }
-            __syncthreads();
-        }
+        if (check) later_check(a, part, nb, it, S);
     }
     for (int i = gtid; i < n; i += gs) {
         const V3<T> x = load3(a.x, i);
@@ -304,8 +323,186 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.out_iter = it;
-        *a.out_status = done ? 0 : 1;
-        for (int c = 0; c < 3; ++c) { a.out_rr[c] = rr[c]; a.out_bb[c] = bb[c]; }
+        *a.out_status = S.done ? 0 : 1;
+        for (int c = 0; c < 3; ++c) { a.out_rr[c] = S.rr[c]; a.out_bb[c] = S.bb[c]; }
+    }
+}
+
+// The same solve with everything of a row that does not change in its
+// thread's registers: the row's first kHeld entries, D^-1, x, r and d, so
+// that an iteration is one round of gathers of d and the barrier; entries beyond
+// kHeld are read each time.  One warp holds a slice of 32 rows, for all three
+// components (NC 3, the FP32 form: a 16-byte gather per entry from [n][4]) or
+// for one of them (NC 1, FP64, from [3][n]: 15 entries of three components
+// keep a warp's FP64 unit busy for 3 us, of one for 1, and there are enough
+// SMs for three times the warps).
+constexpr int kHeld = 16, kRegThreads = 512;
+
+template <typename T, int NC>
+__device__ __forceinline__ void load_nc(const T *v, int n, int comp, int i, T (&g)[NC]) {
+    if constexpr (NC == 3) {
+        const V3<T> q = load3(v, i);
+        g[0] = q.x; g[1] = q.y; g[2] = q.z;
+    } else {
+        g[0] = v[(size_t)comp * n + i];
+    }
+}
+template <typename T, int NC>
+__device__ __forceinline__ void store_nc(T *v, int n, int comp, int i, const T (&g)[NC]) {
+    if constexpr (NC == 3) store3(v, i, V3<T>{g[0], g[1], g[2]});
+    else v[(size_t)comp * n + i] = g[0];
+}
+
+template <typename T, int NC>
+__global__ void __launch_bounds__(kRegThreads, 1) k_mass_cheb3_reg(const __grid_constant__ Cheb3Args<T> a) {
+    cg::grid_group grid = cg::this_grid();
+    __shared__ double sh[16 * 6];
+    __shared__ Checks S;
+    const int nb = gridDim.x, n = a.n, lane = threadIdx.x & 31;
+    const int slices = (n + 31) >> 5, unit = (int)(threadIdx.x >> 5) * nb + blockIdx.x;
+    const bool mine = unit < slices * (3 / NC);
+    const int comp = NC == 3 || !mine ? 0 : unit / slices, slice = mine ? unit - comp * slices : 0;
+    const int i = 32 * slice + lane;
+    const bool live = mine && i < n;
+    const int w = mine ? __ldg(a.swidth + slice) : 0;
+    const int64_t base = mine ? __ldg(a.sptr + slice) + lane : 0;
+    int c[kHeld];
+    T m[kHeld];
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) {
+        c[k] = k < w ? __ldg(a.scol + base + 32 * k) : 0;
+        m[k] = k < w ? __ldg(a.sval + base + 32 * k) : (T)0;
+    }
+    const T dinv = live ? __ldg(a.dinv + i) : (T)0;
+    // this row of M times v (start: the [n][4] start vector, in either form)
+    auto product = [&](const T *v, bool start, T (&s)[NC]) {
+        T g[kHeld][NC];
+#pragma unroll
+        for (int k = 0; k < kHeld; ++k) {
+#pragma unroll
+            for (int q = 0; q < NC; ++q) g[k][q] = (T)0;
+            if (k < w) {
+                if (NC == 1 && start) g[k][0] = v[4 * (size_t)c[k] + comp];
+                else load_nc<T, NC>(v, n, comp, c[k], g[k]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NC; ++q) s[q] = (T)0;
+#pragma unroll
+        for (int k = 0; k < kHeld; ++k)
+#pragma unroll
+            for (int q = 0; q < NC; ++q) s[q] = fma(m[k], g[k][q], s[q]);
+        for (int k = kHeld; k < w; ++k) {
+            const int ck = __ldg(a.scol + base + 32 * k);
+            const T mk = __ldg(a.sval + base + 32 * k);
+            T h[NC];
+            if (NC == 1 && start) h[0] = v[4 * (size_t)ck + comp];
+            else load_nc<T, NC>(v, n, comp, ck, h);
+#pragma unroll
+            for (int q = 0; q < NC; ++q) s[q] = fma(mk, h[q], s[q]);
+        }
+    };
+    T *d = a.d0, *dn = a.d1;
+    T x[NC], r[NC], di[NC], b[NC];
+    double loc[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < NC; ++q) x[q] = r[q] = di[q] = b[q] = (T)0;
+    {
+        double bs[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) bs[q] = 0.0;
+        const int64_t k1 = live ? a.adj_ptr[i + 1] : 0;
+#pragma unroll 4
+        for (int64_t k = live ? a.adj_ptr[i] : 0; k < k1; ++k) {
+            const int cell = __ldg(a.adj_cell + k);
+            const double wt = 0.25 * __ldg(a.vol + cell);
+            const double *E = a.E_cell + 4 * (size_t)cell;
+#pragma unroll
+            for (int q = 0; q < NC; ++q) bs[q] = bs[q] + wt * __ldg(E + (NC == 1 ? comp : q));
+        }
+        T s[NC];
+        product(a.x, true, s);
+        if (live) {
+#pragma unroll
+            for (int q = 0; q < NC; ++q) {
+                x[q] = a.x[4 * (size_t)i + (NC == 1 ? comp : q)];
+                b[q] = (T)bs[q];
+                r[q] = b[q] - s[q];
+                di[q] = dinv * (T)(1.0 / kTheta) * r[q];
+            }
+            store_nc<T, NC>(d, n, comp, i, di);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const bool own = NC == 3 || comp == q;
+        const T rq = NC == 3 ? r[NC == 3 ? q : 0] : r[0], bq = NC == 3 ? b[NC == 3 ? q : 0] : b[0];
+        loc[q] = own ? (double)rq * (double)rq : 0.0;
+        loc[3 + q] = own ? (double)bq * (double)bq : 0.0;
+    }
+    first_check(a, loc, nb, sh, S);
+    if (S.cold[0] || S.cold[1] || S.cold[2]) {
+#pragma unroll
+        for (int q = 0; q < NC; ++q)
+            if (S.cold[NC == 1 ? comp : q]) {
+                x[q] = (T)0;
+                r[q] = b[q];
+                di[q] = dinv * (T)(1.0 / kTheta) * b[q];
+            }
+        if (live) store_nc<T, NC>(d, n, comp, i, di);
+        grid.sync();
+    }
+    int it = 0;
+    while (!S.done && it < a.max_iter) {
+        ++it;
+        const bool check = it == S.next_check;
+        const T c1 = a.c1[min(it, kCheb) - 1], f = a.c2[min(it, kCheb) - 1] * dinv;
+        T s[NC];
+        product(d, false, s);
+#pragma unroll
+        for (int q = 0; q < NC; ++q) {
+            x[q] += di[q];
+            r[q] -= s[q];
+            di[q] = fma(f, r[q], c1 * di[q]);
+        }
+        if (live) store_nc<T, NC>(dn, n, comp, i, di);
+        T *t = d;
+        d = dn;
+        dn = t;
+        double *part = a.partials + (size_t)(6 + 3 * (it & 1)) * nb;   // read by all before it is written again
+        if (check) {
+            double lr[3], out[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const T rq = NC == 3 ? r[NC == 3 ? q : 0] : r[0];
+                lr[q] = NC == 3 || comp == q ? (double)rq * (double)rq : 0.0;
+            }
+            block_sum_n<3>(lr, sh, out);
+            if (threadIdx.x == 0)
+                for (int k = 0; k < 3; ++k) part[k * nb + blockIdx.x] = out[k];
+        }
+        grid.sync();
+        if (check) later_check(a, part, nb, it, S);
+    }
+    if (live) {
+#pragma unroll
+        for (int q = 0; q < NC; ++q) {
+            const int cq = NC == 1 ? comp : q;
+            const size_t o = 4 * (size_t)i + cq;
+            const double v = (double)x[q] + a.e0[cq];
+            a.x[o] = x[q];
+            if (a.ev) a.ev[o] = v;
+            if (a.evf) a.evf[o] = (float)v;
+            if (cq == 2) {
+                if (a.ev) a.ev[o + 1] = 0.0;
+                if (a.evf) a.evf[o + 1] = 0.0f;
+            }
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.out_iter = it;
+        *a.out_status = S.done ? 0 : 1;
+        for (int c2 = 0; c2 < 3; ++c2) { a.out_rr[c2] = S.rr[c2]; a.out_bb[c2] = S.bb[c2]; }
     }
 }
 
@@ -353,9 +550,18 @@ int solve(const EsolveArgs &e, T *buf, const T *sval, const T *dinv, cudaStream_
         a.c2[k] = (T)(2.0 / kDelta * next);
         rho = next;
     }
+    void *params[] = {&a};
+    // rows in registers where one warp per unit fits the grid (up to 25,900
+    // dofs in FP64, 77,800 in FP32), spread over all SMs; else two blocks per SM
+    // striding over the rows
+    constexpr int NC = sizeof(T) == 8 ? 1 : 3;
+    const int units = (e.n + 31) / 32 * (3 / NC), sms = sm_count();
+    if (units <= kRegThreads / 32 * sms) {
+        const int nb = units < sms ? units : sms, warps = (units + nb - 1) / nb;
+        return (int)cudaLaunchCooperativeKernel((const void *)k_mass_cheb3_reg<T, NC>, dim3(nb), dim3(32 * warps), params, 0, st);
+    }
     int blocks = 0, threads = 0;
     launch_shape<T>(e.n, blocks, threads);
-    void *params[] = {&a};
     return (int)cudaLaunchCooperativeKernel((const void *)k_mass_cheb3<T>, dim3(blocks), dim3(threads), params, 0, st);
 }
 

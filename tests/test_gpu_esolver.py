@@ -1,6 +1,7 @@
 """The ESolver's Chebyshev iteration against conjugate gradients in 64 bits on
-the same mass matrix: systems smaller than a warp, of both block shapes, rows
-no multiple of a slice, a second solve from the first one's solution."""
+the same mass matrix: systems smaller than a warp, in registers and over both
+block shapes of the other form, rows no multiple of a slice, rows of more entries
+than are held, a second solve from the first one's solution."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -34,11 +35,32 @@ def reference(mesh, phi):
     return out
 
 
+def fans(n):
+    """A probe mesh with the cells around every 40th vertex split at their
+    centroids: rows of up to 39 entries."""
+    ma = meshgen.probe_box(n, 2.0, 0.9)
+    split = np.isin(ma.cells, np.arange(7, ma.n_vertices, 40)).any(1)
+    old = ma.cells[split]
+    new = ma.n_vertices + np.arange(len(old))
+    parts = []
+    for k in range(4):
+        part = old.copy()
+        part[:, k] = new
+        parts.append(part)
+    coords = np.concatenate([ma.coords, ma.coords[old].mean(1)])
+    return meshgen.MeshArrays(coords=coords, cells=np.concatenate([ma.cells[~split]] + parts), bfacets=ma.bfacets,
+                              btags=ma.btags.copy(), vertex_to_dof=None, n_dofs=len(coords), Ld=ma.Ld,
+                              origin=ma.origin, n_objects=ma.n_objects)
+
+
 @pytest.mark.parametrize("prec", [L.PG_FP64, L.PG_MIXED])
-@pytest.mark.parametrize("geom,n", [("periodic", 2), ("periodic", 3), ("probe", 5), ("periodic", 17), ("probe", 34)])
+@pytest.mark.parametrize("geom,n", [("periodic", 2), ("periodic", 3), ("probe", 5), ("fans", 9), ("periodic", 17),
+                                    ("probe", 27), ("probe", 34), ("probe", 43)])
 def test_esolver(lib, prec, geom, n):
-    ma = meshgen.langmuir_cube(n) if geom == "periodic" else meshgen.probe_box(n, 2.0, 0.9)
+    ma = fans(n) if geom == "fans" else meshgen.langmuir_cube(n) if geom == "periodic" else meshgen.probe_box(n, 2.0, 0.9)
     mesh = punc.Mesh(ma)
+    if geom == "fans":
+        assert np.diff(mesh.table(L.T_CSR_ROWPTR)).max() > 24
     pop = punc.Population(mesh, precision=prec, periodic=geom == "periodic")
     E = punc.Function(pop, "E_cg1")
     es = punc.ESolver(pop)
