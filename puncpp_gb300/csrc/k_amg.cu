@@ -245,16 +245,21 @@ struct FmtH32 {   // binary16 values, 32-bit columns
 };
 
 // The sum over the stored entries of a SELL row: w chunks from off, C of them
-// and their gathers in flight together.
+// and their gathers in flight together, the first C loaded by the caller.
 template <class F, int C>
-__device__ __forceinline__ float sell_sum(const SpOp &S, const float *x, int off, int w, int cb) {
+__device__ __forceinline__ void sell_load(const SpOp &S, int off, int w, F (&f)[C]) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        f[c] = F{};
+        if (c < w) f[c].load(S, off + 32 * c);
+    }
+}
+template <class F, int C>
+__device__ __forceinline__ float sell_sum(const SpOp &S, const float *x, int off, int w, int cb, F (&f)[C]) {
     float sum = 0.0f;
     for (int k = 0; k < w; k += C) {
-        F f[C];
         float g[C][4];
-#pragma unroll
-        for (int c = 0; c < C; ++c)
-            if (k + c < w) f[c].load(S, off + 32 * (k + c));
+        if (k > 0) sell_load(S, off + 32 * k, w - k, f);
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
@@ -270,21 +275,18 @@ __device__ __forceinline__ float sell_sum(const SpOp &S, const float *x, int off
 // The off-diagonal entries of a row of A_0, stored as pairs (w of them): the
 // P1 rows of these meshes hold six, and a chunk of four would pad them to
 // eight in the operator that is read twice per iteration.
-template <bool C16>
-__device__ __forceinline__ float a0_sum(const SpOp &A, const float *x, int off, int w, int cb) {
-    constexpr int C = 3;
-    float sum = 0.0f;
-    for (int k = 0; k < w; k += C) {
-        uint2 v[C], c[C];
-        float g[C][2];
+struct A0Pairs {
+    static constexpr int C = 3;
+    uint2 v[C], c[C];   // values and columns
+    __device__ __forceinline__ void load(const SpOp &A, int off, int w, int cb) {
 #pragma unroll
         for (int q = 0; q < C; ++q) {
             v[q] = make_uint2(0, 0);
             c[q] = make_uint2(0, 0);
-            if (k + q < w) {
-                const int o = off + 32 * (k + q);
+            if (q < w) {
+                const int o = off + 32 * q;
                 v[q] = ld_nc_64((const uint2 *)A.val + o);
-                if (C16) {
+                if (A.c16) {
                     const uint32_t u = ld_nc_32((const uint32_t *)A.col + o);
                     c[q] = make_uint2(cb + (u & 0xffffu), cb + (u >> 16));
                 } else {
@@ -292,15 +294,23 @@ __device__ __forceinline__ float a0_sum(const SpOp &A, const float *x, int off, 
                 }
             }
         }
+    }
+};
+__device__ __forceinline__ float a0_sum(const SpOp &A, const float *x, int off, int w, int cb, A0Pairs &e) {
+    constexpr int C = A0Pairs::C;
+    float sum = 0.0f;
+    for (int k = 0; k < w; k += C) {
+        float g[C][2];
+        if (k > 0) e.load(A, off + 32 * k, w - k, cb);
 #pragma unroll
         for (int q = 0; q < C; ++q) {
-            g[q][0] = k + q < w ? x[c[q].x] : 0.0f;
-            g[q][1] = k + q < w ? x[c[q].y] : 0.0f;
+            g[q][0] = k + q < w ? x[e.c[q].x] : 0.0f;
+            g[q][1] = k + q < w ? x[e.c[q].y] : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < C; ++q) {
-            sum = fmaf(__uint_as_float(v[q].x), g[q][0], sum);
-            sum = fmaf(__uint_as_float(v[q].y), g[q][1], sum);
+            sum = fmaf(__uint_as_float(e.v[q].x), g[q][0], sum);
+            sum = fmaf(__uint_as_float(e.v[q].y), g[q][1], sum);
         }
     }
     return sum;
@@ -341,7 +351,9 @@ __device__ __forceinline__ void product_f(const SpOp &S, const float *x, E &e, S
             const int off = h.off(i), w = h.width(), cb = h.h.y;
             h.load(S, i + st, i1);
             const typename E::Pre pv = e.pre(i);
-            e.row(i, sell_sum<F, 3>(S, x, off, w, cb), pv);
+            F f[3];
+            sell_load(S, off, w, f);
+            e.row(i, sell_sum(S, x, off, w, cb, f), pv);
         }
         return;
     }
@@ -452,52 +464,95 @@ struct DirectRow {
 // this thread's share of r.z: both products of a row in one pass (no vector
 // t_0 = W_0 r to write and read).  omega D^-1 a_ii s_i = omega s_i, so A_0's
 // diagonal is not read.
-template <bool C16, class F>
-__device__ __forceinline__ DF prolong_rows(const SpOp &A, const SpOp &S, const float *s, const float *y, const float *r,
-                                           const float *dinv, float om, float *z, int i0, int i1, int gst) {
-    DF rz{0.0f, 0.0f};
+// kAhead: the operands of a thread's first row that no other thread changes (the
+// operators' heads and entries, s and r of its own) are loaded by first() before
+// the barrier, which ends with the L1 empty: two of the phase's three trips to
+// the L2 then pass while the block waits.  That needs 128 registers, so it is
+// the form of one block per SM (39,298 rows, 10 CG1 steps 5.41 -> 5.12 ms; 68,908
+// rows, solve 0.60 -> 0.56 ms); in 64 registers it spills, and in a cluster, whose
+// barrier is short, it gained nothing (4,096 rows 1% slower).
+template <class F, bool kAhead>
+struct Prolong {
     SellHead ha, hs;
-    ha.load(A, i0, i1);
-    hs.load(S, i0, i1);
-    for (int i = i0; i < i1; i += gst) {
-        const int oa = ha.off(i), wa = ha.width(), ca = ha.h.y, os = hs.off(i), ws = hs.width(), cs = hs.h.y;
-        ha.load(A, i + gst, i1);
-        hs.load(S, i + gst, i1);
-        const float si = s[i], ri = r[i], di = __ldg(dinv + i);
-        const float q = a0_sum<C16>(A, s, oa, wa, ca);
-        const float u = sell_sum<F, 3>(S, y, os, ws, cs);
-        const float v = fmaf(-om * di, q, (2.0f - om) * si) + u;
-        z[i] = v;
-        rz = df_fma(v, ri, rz);
+    A0Pairs ea;
+    F es[3];
+    float si = 0.0f, ri = 0.0f, di = 0.0f;
+    __device__ __forceinline__ void load(const SpOp &A, const float *s, const float *r, const float *dinv, int i) {
+        si = s[i]; ri = r[i]; di = __ldg(dinv + i);
+        ea.load(A, ha.off(i), ha.width(), ha.h.y);
     }
-    return rz;
-}
+    __device__ __forceinline__ void first(const SpOp &A, const SpOp &S, const float *s, const float *r, const float *dinv, int i0, int i1) {
+        if (!kAhead) return;
+        ha.load(A, i0, i1);
+        hs.load(S, i0, i1);
+        if (i0 < i1) {
+            load(A, s, r, dinv, i0);
+            sell_load(S, hs.off(i0), hs.width(), es);
+        }
+    }
+    __device__ __forceinline__ DF rows(const SpOp &A, const SpOp &S, const float *s, const float *y, const float *r,
+                                       const float *dinv, float om, float *z, int i0, int i1, int st) {
+        DF rz{0.0f, 0.0f};
+        if (!kAhead) {
+            ha.load(A, i0, i1);
+            hs.load(S, i0, i1);
+        }
+        for (int i = i0; i < i1; i += st) {
+            const bool have = kAhead && i == i0;
+            if (!have) load(A, s, r, dinv, i);
+            const int oa = ha.off(i), wa = ha.width(), ca = ha.h.y, os = hs.off(i), ws = hs.width(), cs = hs.h.y;
+            ha.load(A, i + st, i1);
+            hs.load(S, i + st, i1);
+            const float q = a0_sum(A, s, oa, wa, ca, ea);
+            if (!have) sell_load(S, os, ws, es);
+            const float u = sell_sum(S, y, os, ws, cs, es);
+            const float v = fmaf(-om * di, q, (2.0f - om) * si) + u;
+            z[i] = v;
+            rz = df_fma(v, ri, rz);
+        }
+        return rz;
+    }
+};
 
-// p = z + beta p, Ap = A z + beta Ap (beta 0 and no reads of p, Ap on the
-// first step), and this thread's shares of p.Ap, r.Ap and Ap.Ap.
-template <bool C16>
-__device__ __forceinline__ void direction_rows(const SpOp &A, const float *diag, const float *z, const float *r,
-                                               float *p, float *Ap, float beta, bool first, DF (&v)[3], int i0, int i1, int gst) {
-    float pap = 0.0f, rap = 0.0f, apap = 0.0f;
+// p = z + beta p, Ap = A z + beta Ap (none: the
+// first step, no reads of p and Ap), and this thread's shares of p.Ap, r.Ap and Ap.Ap.
+template <bool kAhead>
+struct Direction {
     SellHead h;
-    h.load(A, i0, i1);
-    for (int i = i0; i < i1; i += gst) {
-        const int off = h.off(i), w = h.width(), cb = h.h.y;
-        h.load(A, i + gst, i1);
-        const float zi = z[i], ri = r[i], di = __ldg(diag + i);
-        const float p0 = first ? 0.0f : p[i], q0 = first ? 0.0f : Ap[i];
-        const float s = fmaf(di, zi, a0_sum<C16>(A, z, off, w, cb));
-        const float pi = fmaf(beta, p0, zi), api = fmaf(beta, q0, s);
-        p[i] = pi;
-        Ap[i] = api;
-        pap = fmaf(pi, api, pap);
-        rap = fmaf(ri, api, rap);
-        apap = fmaf(api, api, apap);
+    A0Pairs e;
+    float di = 0.0f;
+    __device__ __forceinline__ void load(const SpOp &A, const float *diag, int i) {
+        e.load(A, h.off(i), h.width(), h.h.y);
+        di = __ldg(diag + i);
     }
-    v[0] = DF{pap, 0.0f};
-    v[1] = DF{rap, 0.0f};
-    v[2] = DF{apap, 0.0f};
-}
+    __device__ __forceinline__ void first(const SpOp &A, const float *diag, int i0, int i1) {
+        if (!kAhead) return;
+        h.load(A, i0, i1);
+        if (i0 < i1) load(A, diag, i0);
+    }
+    __device__ __forceinline__ void rows(const SpOp &A, const float *diag, const float *z, const float *r, float *p,
+                                         float *Ap, float beta, bool none, DF (&v)[3], int i0, int i1, int st) {
+        float pap = 0.0f, rap = 0.0f, apap = 0.0f;
+        if (!kAhead) h.load(A, i0, i1);
+        for (int i = i0; i < i1; i += st) {
+            if (!kAhead || i != i0) load(A, diag, i);
+            const int off = h.off(i), w = h.width(), cb = h.h.y;
+            h.load(A, i + st, i1);
+            const float zi = z[i], ri = r[i];
+            const float p0 = none ? 0.0f : p[i], q0 = none ? 0.0f : Ap[i];
+            const float s = fmaf(di, zi, a0_sum(A, z, off, w, cb, e));
+            const float pi = fmaf(beta, p0, zi), api = fmaf(beta, q0, s);
+            p[i] = pi;
+            Ap[i] = api;
+            pap = fmaf(pi, api, pap);
+            rap = fmaf(ri, api, rap);
+            apap = fmaf(api, api, apap);
+        }
+        v[0] = DF{pap, 0.0f};
+        v[1] = DF{rap, 0.0f};
+        v[2] = DF{apap, 0.0f};
+    }
+};
 
 // Blocks [0, cut) take the first and [cut, nb) the second of two independent
 // products of one phase, in proportion to their stored chunks, so that their
@@ -576,9 +631,10 @@ struct CgUpdate {
 // (double-float; a cluster keeps them in shared memory); [4 nb, 6 nb) the FP64 true residual's and right-hand side's
 // squares.  A buffer is written again only after at least one barrier has
 // passed since every block read it.
-template <class Sync>
-__global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constant__ PcgArgs a,
+template <class Sync, int kBlocks>
+__global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_constant__ PcgArgs a,
                                                             const __grid_constant__ AmgDev M) {
+    constexpr bool kAhead = kBlocks == 1;
     __shared__ double sh[2 * kPcgThreads + 16];   // FP64 sums; the double-float ones use its head
     __shared__ DF tot[3];
     __shared__ double scal[2];                    // FP64 scalars; 1: go on
@@ -629,6 +685,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
     float beta = 0.0f;
     // fresh: start a pass, from the FP64 true residual; else a CG step
     bool fresh = true;
+    Direction<kAhead> dir;
     for (;;) {
         bool keep = false;
         if (fresh) {
@@ -670,8 +727,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             // ||r - alpha Ap||^2 = ||r||^2 - 2 alpha r.Ap + alpha^2 Ap.Ap, which
             // only decides when the residual is replaced
             DF v[3];
-            if (M.lev[0].A.c16) direction_rows<true>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
-            else direction_rows<false>(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
+            dir.rows(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
             CgUpdate up;
             up.load(a, i0, i1, gst);
             block_part<3, Sync>(v, shf, partA, nb);
@@ -748,29 +804,28 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_amg(const __grid_constan
             }
             Sync::sync();
         }
-        if (L >= 2) {
-            AddRow e{M.y1, M.lev[1].t};
-            product<true>(M.U1, M.stack, e, all);
-            if (keep) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
-            Sync::sync();
-            yup = M.y1;
-        }
         DF v[1];
         if (L >= 1) {
             const SpOp &A0 = M.lev[0].A;
-            if (A0.c16 && M.S0.c16)
-                v[0] = prolong_rows<true, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
-            else if (M.S0.c16)
-                v[0] = prolong_rows<false, FmtH16>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
-            else if (A0.c16)
-                v[0] = prolong_rows<true, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
-            else
-                v[0] = prolong_rows<false, FmtH32>(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
+            if (L >= 2) {
+                AddRow e{M.y1, M.lev[1].t};
+                product<true>(M.U1, M.stack, e, all);
+                if (keep) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
+                yup = M.y1;
+            }
+            auto up = [&](auto pro) {
+                pro.first(A0, M.S0, s0, r, a.dinv32, i0, i1);
+                if (L >= 2) Sync::sync();
+                v[0] = pro.rows(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
+            };
+            if (M.S0.c16) up(Prolong<FmtH16, kAhead>{});
+            else up(Prolong<FmtH32, kAhead>{});
         } else {
             DirectRow e{z, r, DF{0.0f, 0.0f}};
             product<false>(M.cinv, r, e, all);
             v[0] = e.rz;
         }
+        dir.first(M.lev[0].A, M.diag0, i0, i1);
         block_part<1, Sync>(v, shf, partC, nb);
         Sync::sync();
         grid_total<1, Sync>(partC, nb, t_rz + (it & 1));
@@ -834,7 +889,7 @@ int pcg_amg_grid_blocks() {
     static int g = 0;
     if (g == 0) {
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_amg<GridSync>, kPcgThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_amg<GridSync, 2>, kPcgThreads, 0);
         if (per_sm < 1) per_sm = 1;
         if (per_sm > 2) per_sm = 2;
         g = per_sm * sm_count();
@@ -846,7 +901,7 @@ int pcg_amg_grid_blocks() {
 static int cluster_blocks() {
     static int g = 0;
     if (g == 0) {
-        const void *fn = (const void *)k_pcg_amg<ClusterSync>;
+        const void *fn = (const void *)k_pcg_amg<ClusterSync, 2>;
         int best = 1;
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
         for (int k = kClusterMax; k > 1; k /= 2) {
@@ -886,7 +941,7 @@ int launch_pcg_amg(const PcgArgs &a, const AmgDev &amg, cudaStream_t st) {
         cfg.stream = st;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        return (int)cudaLaunchKernelExC(&cfg, (const void *)k_pcg_amg<ClusterSync>, params);
+        return (int)cudaLaunchKernelExC(&cfg, (const void *)k_pcg_amg<ClusterSync, 2>, params);
     }
     int nb = pcg_amg_grid_blocks();
     // one row per thread where the blocks suffice; below one block per SM twice
@@ -895,7 +950,8 @@ int launch_pcg_amg(const PcgArgs &a, const AmgDev &amg, cudaStream_t st) {
     // rows 0.56 ms with 43, 0.55 with 86, 0.60 with 152)
     const int need = (a.n + kPcgThreads - 1) / kPcgThreads, sms = sm_count();
     if (need < nb) nb = need > sms ? need : std::max(need, std::min(sms, 2 * need));
-    return (int)cudaLaunchCooperativeKernel((const void *)k_pcg_amg<GridSync>, dim3(nb), dim3(kPcgThreads), params, 0, st);
+    const void *fn = nb <= sms ? (const void *)k_pcg_amg<GridSync, 1> : (const void *)k_pcg_amg<GridSync, 2>;
+    return (int)cudaLaunchCooperativeKernel(fn, dim3(nb), dim3(kPcgThreads), params, 0, st);
 }
 
 }  // namespace pg
