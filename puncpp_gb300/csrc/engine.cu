@@ -160,6 +160,16 @@ struct pg_sim {
     // reductions, state
     DevState *state = nullptr;
     DevState *state_h = nullptr;   // pinned
+    // pinned: what the calls that wait for a result read back, one copy each (a
+    // copy to pageable memory is staged and waited for in the call: 10 us
+    // each, two per solve and up to twelve in a step of separate calls)
+    struct ReadBack {
+        double pcg_d[2];
+        int32_t pcg_i[2];
+        double es_d[6];
+        int32_t es_i[2];
+        double ke, pe;
+    } *read_h = nullptr;
     double *partials = nullptr, *ke_dev = nullptr;
     int n_part = 0;                           // blocks of a particle pass (partial sums in use)
     int part_cap = 0;                         // partial-sum slots allocated
@@ -187,6 +197,11 @@ namespace {
         if (e_ != cudaSuccess)                                                                 \
             return fail(PG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
     } while (0)
+
+// The solvers' results in one buffer each: the FP64 values, then two integers.
+constexpr size_t kPcgOutBytes = 2 * sizeof(double) + 2 * sizeof(int32_t);
+constexpr size_t kEsOutBytes = 6 * sizeof(double) + 2 * sizeof(int32_t);
+static_assert(sizeof(pg_sim::ReadBack) == kPcgOutBytes + kEsOutBytes + 2 * sizeof(double), "packed as on the device");
 
 template <class T>
 int dalloc(pg_sim *s, T **p, size_t count) {
@@ -778,11 +793,10 @@ static int poisson_solve_internal(pg_sim *s, const double *pot_h, bool zero_rho,
         e = s->use_amg ? launch_pcg_amg(a, s->amg, s->stream) : launch_pcg(a, s->stream);
     }
     if (e) return fail(PG_ERR_CUDA, std::string("cooperative PCG launch: ") + cudaGetErrorString((cudaError_t)e));
-    int32_t oi[2];
-    double od[2];
-    PG_CUDA(cudaMemcpyAsync(oi, s->pcg_out_i, sizeof(oi), cudaMemcpyDeviceToHost, s->stream));
-    PG_CUDA(cudaMemcpyAsync(od, s->pcg_out_d, sizeof(od), cudaMemcpyDeviceToHost, s->stream));
+    PG_CUDA(cudaMemcpyAsync(s->read_h->pcg_d, s->pcg_out_d, kPcgOutBytes, cudaMemcpyDeviceToHost, s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    const int32_t *oi = s->read_h->pcg_i;
+    const double *od = s->read_h->pcg_d;
     *valid = true;
     if (acc) {
         acc->iterations += oi[0];
@@ -1289,9 +1303,10 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
         const int nb = std::max(pcg_grid_blocks(), 2 * pcg_amg_grid_blocks());
         if ((rc = dalloc(s, &s->r, nd)) || (rc = dalloc(s, &s->z, nd)) || (rc = dalloc(s, &s->p0, nd)) ||
             (rc = dalloc(s, &s->p1, nd)) || (rc = dalloc(s, &s->Ap, nd)) || (rc = dalloc(s, &s->pcg_part, 4 * nb)) ||
-            (rc = dalloc(s, &s->pcg_out_i, 2)) || (rc = dalloc(s, &s->pcg_out_d, 2)) ||
+            (rc = dalloc(s, &s->pcg_out_d, kPcgOutBytes / sizeof(double))) ||
             (rc = dalloc(s, &s->obj_pot, std::max(1, s->n_obj))) || (rc = dalloc(s, &s->image, std::max(1, s->n_obj))))
             return bail(rc);
+        s->pcg_out_i = reinterpret_cast<int32_t *>(s->pcg_out_d + 2);
         if (cfg.pcg_precond != 0 && cfg.pcg_precond != 1) return bail(fail(PG_ERR_ARG, "pg_create: unknown pcg_precond"));
         const bool amg = cfg.pcg_precond == 0;
         const int mode = amg ? 2 : (cfg.pcg_precision == 0 ? (cfg.precision == PG_MIXED ? 2 : 1) : cfg.pcg_precision);
@@ -1326,9 +1341,10 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
                 if (h.col[k] == i && h.M[k] != 0.0) mdinv[i] = 1.0 / h.M[k];
         if ((rc = upload(s, &s->es_adj_ptr, aptr)) || (rc = upload(s, &s->es_adj_cell, acell)) ||
             (rc = upload(s, &s->es_vol, h.volume)) || (rc = upload(s, &s->M_dinv, mdinv)) ||
-            (rc = dalloc(s, &s->es_part, 12 * std::max(1, esolve_grid_blocks()))) || (rc = dalloc(s, &s->es_out_i, 2)) ||
-            (rc = dalloc(s, &s->es_out_d, 6)) || (rc = dalloc(s, &s->Ev, 4 * nd)))
+            (rc = dalloc(s, &s->es_part, 12 * std::max(1, esolve_grid_blocks()))) || (rc = dalloc(s, &s->es_out_d, kEsOutBytes / sizeof(double))) ||
+            (rc = dalloc(s, &s->Ev, 4 * nd)))
             return bail(rc);
+        s->es_out_i = reinterpret_cast<int32_t *>(s->es_out_d + 6);
         cudaMemset(s->Ev, 0, sizeof(double) * 4 * nd);
         if (cfg.precision == PG_MIXED) {
             std::vector<float> d32(mdinv.begin(), mdinv.end());
@@ -1381,7 +1397,9 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
     // state, reductions, sort scratch
     if ((rc = dalloc(s, &s->state, 1))) return bail(rc);
     cudaMemset(s->state, 0, sizeof(DevState));
-    if (cudaMallocHost(&s->state_h, sizeof(DevState)) != cudaSuccess) return bail(fail(PG_ERR_CUDA, "cudaMallocHost failed"));
+    if (cudaMallocHost(&s->state_h, sizeof(DevState)) != cudaSuccess ||
+        cudaMallocHost(&s->read_h, sizeof(pg_sim::ReadBack)) != cudaSuccess)
+        return bail(fail(PG_ERR_CUDA, "cudaMallocHost failed"));
     std::memset(s->state_h, 0, sizeof(DevState));
     s->n_part = sm_count() * 8;
     s->part_cap = sm_count() * 32;
@@ -1415,6 +1433,7 @@ int pg_destroy(pg_sim *s) {
     if (s->inj_offsets) cudaFree(s->inj_offsets);
     if (s->scan_tmp) cudaFree(s->scan_tmp);
     if (s->state_h) cudaFreeHost(s->state_h);
+    if (s->read_h) cudaFreeHost(s->read_h);
     for (auto &e : s->ev_pending) { cudaEventDestroy(e.second.first); cudaEventDestroy(e.second.second); }
     for (auto &e : s->user_ev)
         if (e) cudaEventDestroy(e);
@@ -1716,11 +1735,10 @@ static int esolver_internal(pg_sim *s, const double E0[3], pg_solve_info *info) 
         err = launch_esolve(e, s->stream);
     }
     if (err) return fail(PG_ERR_CUDA, std::string("ESolver launch: ") + cudaGetErrorString((cudaError_t)err));
-    int32_t oi[2];
-    double od[6];
-    PG_CUDA(cudaMemcpyAsync(oi, s->es_out_i, sizeof(oi), cudaMemcpyDeviceToHost, s->stream));
-    PG_CUDA(cudaMemcpyAsync(od, s->es_out_d, sizeof(od), cudaMemcpyDeviceToHost, s->stream));
+    PG_CUDA(cudaMemcpyAsync(s->read_h->es_d, s->es_out_d, kEsOutBytes, cudaMemcpyDeviceToHost, s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    const int32_t *oi = s->read_h->es_i;
+    const double *od = s->read_h->es_d;
     if (info) {
         info->iterations = oi[0];
         info->solves = 1;
@@ -1782,8 +1800,9 @@ int pg_potential_energy(pg_sim *s, double *PE) {
     int rc = diag_scratch(s);
     if (rc) return rc;
     launch_potential_energy(s->dm, s->P[s->cur], s->n_slots, is_mixed(s), s->d_q, s->phi, s->diag_acc, s->stream);
-    PG_CUDA(cudaMemcpyAsync(PE, s->diag_acc, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    PG_CUDA(cudaMemcpyAsync(&s->read_h->pe, s->diag_acc, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    *PE = s->read_h->pe;
     return PG_OK;
 }
 
@@ -1898,10 +1917,9 @@ static int push_common(pg_sim *s, const double *B, double dt, bool accel, double
         } else {
             launch_push(s->dm, s->P[s->cur], s->n_slots, pp, s->partials, s->n_part, s->ke_dev, s->stream);
         }
-        double ke = 0;
-        PG_CUDA(cudaMemcpyAsync(&ke, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+        PG_CUDA(cudaMemcpyAsync(&s->read_h->ke, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         PG_CUDA(cudaStreamSynchronize(s->stream));
-        if (KE) *KE = ke;
+        if (KE) *KE = s->read_h->ke;
     } else if (KE) {
         *KE = 0.0;
     }
@@ -1994,8 +2012,9 @@ int pg_kinetic_energy(pg_sim *s, double *KE) {
     } else {
         launch_kinetic(s->P[s->cur], s->n_slots, hm, s->partials, s->n_part, s->ke_dev, s->stream);
     }
-    PG_CUDA(cudaMemcpyAsync(KE, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    PG_CUDA(cudaMemcpyAsync(&s->read_h->ke, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    *KE = s->read_h->ke;
     return PG_OK;
 }
 
@@ -3077,7 +3096,7 @@ int pg_step(pg_sim *s, const pg_step_args *a, pg_object *objects, int32_t n_obje
         StageScope t(s, "PE");
         if ((rc = diag_scratch(s))) return rc;
         launch_potential_energy(s->dm, s->P[s->cur], s->n_slots, is_mixed(s), s->d_q, s->phi, s->diag_acc, s->stream);
-        PG_CUDA(cudaMemcpyAsync(&out.PE, s->diag_acc, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+        PG_CUDA(cudaMemcpyAsync(&s->read_h->pe, s->diag_acc, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     }
     // accelerator + move + update, depositing the next step's charge
     {
@@ -3108,11 +3127,11 @@ int pg_step(pg_sim *s, const pg_step_args *a, pg_object *objects, int32_t n_obje
                               s->state, s->partials, s->n_part, s->ke_dev, s->stream);
         else if (s->n_slots == 0)
             PG_CUDA(cudaMemsetAsync(s->ke_dev, 0, sizeof(double), s->stream));
-        double ke = 0;
-        PG_CUDA(cudaMemcpyAsync(&ke, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+        PG_CUDA(cudaMemcpyAsync(&s->read_h->ke, s->ke_dev, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         rc = check_state(s);
         if (rc) return rc;
-        out.KE = ke;
+        out.KE = s->read_h->ke;
+        if (a->potential_energy) out.PE = s->read_h->pe;
         absorbed_to_objects(s, objects, n_objects, a->dt, &out.n_absorbed);
     }
     if (a->inject) {
