@@ -432,7 +432,8 @@ typedef struct pg_poisson_layout {
     int64_t cycle_nnz_g;                     /* entries of G = C^-1 S^T (last restriction + coarse solve) */
     int64_t cycle_nnz_u1;                    /* entries of the collapsed up-sweep operator of levels >= 1 */
     int64_t cycle_bytes;                     /* operator bytes one AMG-PCG iteration reads: stored entries
-                                                (padding excluded) times their stored size, each operator
+                                                (padding excluded; A_0's diagonal, kept apart, as
+                                                entries) times their stored size, each operator
                                                 counted once per use */
 } pg_poisson_layout;
 int pg_poisson_layout_get(pg_sim *sim, pg_poisson_layout *out);

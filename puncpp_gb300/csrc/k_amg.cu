@@ -1,5 +1,5 @@
 // PCG preconditioned by one smoothed-aggregation AMG V-cycle per iteration,
-// all in one cooperative launch.
+// all in one launch (a cooperative grid, or one thread-block cluster).
 //
 // Krylov recurrence in FP32 with the solution and the true-residual
 // replacements in FP64, inner products of FP32 values summed in double-float
@@ -29,9 +29,11 @@
 // stored with it (s, AmgLevelDev::sb).
 //
 // What bounds it: the chain of dependent loads of each phase (entries, then
-// gathers) and the barriers.  Solves (GB300), before -> after this form: 80^3
-// probe (531k rows) 1.63 -> 1.28 ms, 56^3 (185k) 1.10 -> 0.79, 16^3 periodic (4096)
-// 0.69 -> 0.43.
+// gathers) and the barriers; at 80^3 also the L2, at 4 to 4.5 TB/s in the two
+// phases that stream the level-0 operators.  Solves (GB300), before this form ->
+// with it -> with the cluster form, sums without divergent shuffles, spread rows
+// and operands loaded ahead: 80^3 probe (531k rows) 1.63 -> 1.28 -> 1.21 ms, 56^3
+// (185k) 1.10 -> 0.79 -> 0.74, 16^3 periodic (4096) 0.69 -> 0.43 -> 0.28.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
