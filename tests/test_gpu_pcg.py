@@ -57,13 +57,17 @@ def test_probe_solve(lib, n, order):
     pop.close()
 
 
-@pytest.mark.parametrize("n", [24, 34, 42, 54])
-def test_grid_solve(lib, n):
+@pytest.mark.parametrize("n,order", [(24, "natural"), (34, "natural"), (40, "random"), (42, "natural"),
+                                     (54, "natural")])
+def test_grid_solve(lib, n, order):
     """The grid's forms: two blocks per 512 rows (15k rows), one block per SM
-    (42k), one per 512 rows (79k), more rows than threads (166k), against
+    (42k; 69k in random order, whose columns span more than 16 bits), one per 512
+    rows (79k), more rows than threads (166k), against
     a CG of the host at a residual of 1e-13, with the bound of test_probe_solve."""
     rng = np.random.default_rng(n)
     ma = meshgen.probe_box(n, 2.0, 0.9)
+    if order == "random":
+        ma = renumbered(ma, rng)
     mesh = punc.Mesh(ma)
     K, M = matrices(mesh)
     kind = mesh.table(L.T_BC_KIND)
