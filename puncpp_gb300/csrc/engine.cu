@@ -1174,17 +1174,11 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
     if ((rc = upload(s, &d_binptr, h.bin_ptr)) || (rc = upload(s, &d_bincells, h.bin_cells))) return bail(rc);
     s->dm.bin_ptr = d_binptr;
     s->dm.bin_cells = d_bincells;
-    {
-        // the cells fill the bounding box (a convex domain without a hole)
-        double vol = 0.0, box = 1.0;
-        for (double v : h.volume) vol += v;
-        for (int j = 0; j < 3; ++j) {
-            box *= h.bbox_hi[j] - h.bbox_lo[j];
-            s->dm.lo_f[j] = (float)h.bbox_lo[j];
-            s->dm.bin_inv_f[j] = (float)(1.0 / h.bin_h[j]);
-        }
-        s->dm.box = std::fabs(vol - box) <= 1e-9 * box && cfg.max_walk_steps >= kBoxWalkLimit ? 1 : 0;
+    for (int j = 0; j < 3; ++j) {
+        s->dm.lo_f[j] = (float)h.bbox_lo[j];
+        s->dm.bin_inv_f[j] = (float)(1.0 / h.bin_h[j]);
     }
+    s->dm.box = cfg.max_walk_steps >= kBoxWalkLimit && box_span(h) > 0 ? 1 : 0;
 
     // fields
     if ((rc = dalloc(s, &s->rho_acc, h.ndof)) || (rc = dalloc(s, &s->rho, h.ndof)) || (rc = dalloc(s, &s->phi, h.ndof)) ||

@@ -462,6 +462,47 @@ int build_mesh(const pg_mesh_desc *d, double eps0, HostMesh &h) {
     return PG_OK;
 }
 
+// A plate of no thickness, a hole of any size and a second component all have
+// facets without a neighbour inside the bounding box, so the facets are looked
+// at and not the volume alone.  The volume tells a box that is covered once.
+int64_t box_span(const HostMesh &h) {
+    double vol = 0.0, box = 1.0;
+    for (double v : h.volume) vol += v;
+    for (int j = 0; j < 3; ++j) box *= h.bbox_hi[j] - h.bbox_lo[j];
+    if (!(std::fabs(vol - box) <= 1e-9 * box)) return 0;
+    for (int64_t c = 0; c < h.nc; ++c)
+        for (int f = 0; f < 4; ++f) {
+            if (h.nbr[4 * c + f] >= 0) continue;
+            bool wall = false;
+            for (int j = 0; j < 3 && !wall; ++j) {
+                bool lo = true, hi = true;
+                for (int i = 0; i < 4; ++i) {
+                    if (i == f) continue;
+                    const double x = h.coords[3 * h.cell_vertices[4 * c + i] + j];
+                    lo = lo && x == h.bbox_lo[j];
+                    hi = hi && x == h.bbox_hi[j];
+                }
+                wall = lo || hi;
+            }
+            if (!wall) return 0;
+        }
+    // breadth first from cell 0
+    std::vector<char> seen(h.nc, 0);
+    std::vector<int32_t> front{0}, next;
+    seen[0] = 1;
+    int64_t reached = 0, span = -1;
+    for (; !front.empty(); front.swap(next), ++span) {
+        reached += (int64_t)front.size();
+        next.clear();
+        for (int32_t c : front)
+            for (int f = 0; f < 4; ++f) {
+                const int64_t o = h.nbr[4 * (int64_t)c + f];
+                if (o >= 0 && !seen[o]) { seen[o] = 1; next.push_back((int32_t)o); }
+            }
+    }
+    return reached == h.nc ? std::max<int64_t>(1, span) : 0;
+}
+
 }  // namespace pg
 
 extern "C" {

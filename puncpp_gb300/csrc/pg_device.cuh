@@ -59,8 +59,9 @@ struct DevMesh {
     // point location considers cells in [loc_lo, loc_hi) only (batched runs
     // whose meshes overlap in space)
     int32_t loc_lo = 0, loc_hi = 0x7fffffff;
-    // 1: the cells fill the bounding box, so a walk may start again near its
-    // point (walk_screened); FP32 copies of the bins' origin and 1 / width
+    // 1: the mesh is a box without an inner wall (box_span) and the step limit
+    // is out of a walk's reach, so a walk may start again near its point
+    // (walk_screened); FP32 copies of the bins' origin and 1 / width
     int32_t box = 0;
     float lo_f[3] = {0, 0, 0}, bin_inv_f[3] = {1, 1, 1};
 };

@@ -100,9 +100,9 @@ constexpr int kNearSteps = 256;
 // us with them, 224 without, then 153 with the warp kept together).  R, have_rec: the first cell's record when the
 // caller has it; R and l are the last cell's on return.
 //
-// NEAR: in a mesh whose cells fill their bounding box (m.box; set only with a
-// step limit that no walk through such a mesh reaches) a walk that starts far
-// from its point starts again at a cell near it.  The result counts only if the
+// NEAR: in a box without an inner wall (m.box; set only with a step limit that
+// no walk through such a mesh reaches) a walk that starts far from its point
+// starts again at a cell near it.  The result counts only if the
 // point lies inside its cell by more than the error bounds: that cell is then
 // the only one whose four plane values are not positive, the one where the
 // long walk ends too.  Otherwise the long walk runs.
