@@ -1178,7 +1178,10 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
         s->dm.lo_f[j] = (float)h.bbox_lo[j];
         s->dm.bin_inv_f[j] = (float)(1.0 / h.bin_h[j]);
     }
-    s->dm.box = cfg.max_walk_steps >= kBoxWalkLimit && box_span(h) > 0 ? 1 : 0;
+    {
+        const int64_t span = box_span(h);
+        s->dm.box = span > 0 && cfg.max_walk_steps / kBoxWalkSpans >= span ? 1 : 0;
+    }
 
     // fields
     if ((rc = dalloc(s, &s->rho_acc, h.ndof)) || (rc = dalloc(s, &s->rho, h.ndof)) || (rc = dalloc(s, &s->phi, h.ndof)) ||

@@ -28,9 +28,15 @@ constexpr int kFixedBits = 30;
 constexpr int64_t kMaxMixedSlots = int64_t(1) << (62 - kFixedBits);
 constexpr int kDead = -1;                 // cell id of a free particle slot
 constexpr int kWalkFail = -2147483647;    // walk step limit reached
-// step limit from which a walk may start again near its point (DevMesh::box):
-// a walk crosses a box of 2^31 cells in fewer steps
-constexpr int kBoxWalkLimit = 65536;
+// DevMesh::box is set for a step limit of at least this many spans of the box
+// (box_span), which a walk through it does not reach, so that a walk that ends
+// with the limit's error does so with and without a restart.  In a box cut by
+// whole planes (Kuhn cells) each step of a walk crosses one of the planes between
+// its cell and its point, and none twice: it takes no more steps than lie
+// between two cells, at most two spans.  The rest is for cells of other
+// shapes.  (A walk that never ends, which cells cut against the Delaunay
+// condition allow, is an error without a restart and may find its cell with it.)
+constexpr int kBoxWalkSpans = 8;
 
 struct DevMesh {
     int32_t nc = 0, ndof = 0;

@@ -1,6 +1,6 @@
 """Meshes whose cells fill their bounding box, or all but a trace of it, though
 walls stand inside: a plate of no thickness, an object of a billionth of the
-volume, two boxes side by side."""
+volume, two boxes side by side; and a slender box."""
 import numpy as np
 
 from puncpp_gb300 import meshgen
@@ -60,3 +60,15 @@ def side_by_side(n=6):
     coords = np.concatenate([a.coords, b.coords + [1.0, 0.0, 0.0]])
     cells = np.concatenate([a.cells, b.cells + a.n_vertices])
     return _arrays(coords, cells, lambda fx: np.ones(len(fx)), 0), a.n_cells
+
+
+def slender(n):
+    """Box of 1 x 1 x n unit cubes."""
+    corner = np.array([[i, j, k] for i in (0, 1) for j in (0, 1) for k in (0, 1)])
+    cube = meshgen._kuhn_cells(1)
+    ids = np.empty((n, 8), np.int64)
+    for v, (i, j, k) in enumerate(corner):
+        ids[:, v] = 4 * (np.arange(n) + k) + 2 * i + j
+    z = np.repeat(np.arange(n + 1), 4)
+    coords = np.stack([np.tile([0, 0, 1, 1], n + 1), np.tile([0, 1, 0, 1], n + 1), z], axis=1).astype(float)
+    return _arrays(coords, ids[:, cube].reshape(-1, 4), lambda fx: np.ones(len(fx)), 0)

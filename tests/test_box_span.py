@@ -55,3 +55,7 @@ def test_span_of_a_box(span, n):
     f = np.stack([c[:, 0], c[:, 1], c[:, 2], c[:, 0] - c[:, 1], c[:, 0] - c[:, 2], c[:, 1] - c[:, 2]])
     far = np.abs(np.floor(f) - np.floor(f[:, :1])).sum(axis=0).max()
     assert span(ma) == max(1, far)
+
+
+def test_span_of_a_slender_box(span):
+    assert 3 * 300 - 3 <= span(box_meshes.slender(300)) <= 3 * 300 + 3

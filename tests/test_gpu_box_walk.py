@@ -1,6 +1,6 @@
 """Walks of Population::update in meshes that fill their bounding box though
 walls stand inside, against pg_relocate's walk through every cell between: no
-particle may pass a wall."""
+particle may pass a wall.  And the step limit in a slender box."""
 import numpy as np
 import pytest
 
@@ -67,3 +67,22 @@ def test_boxes_side_by_side(lib, prec):
     to = x + np.array([1.75, 0.0, 0.0])
     want = crossing(ma, prec, x, to, [])
     assert (want == -1).all()
+
+
+@pytest.mark.parametrize("prec", FORMS)
+def test_walk_limit_of_a_slender_box(lib, prec):
+    """120,000 cells between the ends, 100,000 the default limit."""
+    n = 40000
+    pop = punc.Population(punc.Mesh(box_meshes.slender(n)), precision=prec, pcg_precond=1)
+    x = np.array([[0.3, 0.6, 0.5], [0.3, 0.6, 0.5]])
+    to = np.array([[0.4, 0.5, 20000.25], [0.4, 0.5, n - 0.25]])
+    assert pop.add_particles(x[:1], to[:1] - x[:1], -1.0, 1.0) == 1
+    punc.move(pop, 1.0)
+    pop.update([], 1.0)
+    assert pop.num_of_particles() == 1
+    assert pop.add_particles(x[1:], to[1:] - x[1:], -1.0, 1.0) == 1
+    punc.move(pop, 1.0)
+    with pytest.raises(L.PgError) as e:
+        pop.update([], 1.0)
+    assert e.value.code == 5
+    pop.close()
