@@ -159,14 +159,18 @@ __device__ __forceinline__ int iterations_left(double rr, double tol2, float sla
 }
 
 // What the blocks decide together, each for itself from the same sums.
+// bad: a residual or right-hand side that is not finite (or whose square is
+// not), which ends the solve as not converged.
 struct Checks {
     double tol2[3], rr[3], bb[3];
-    int next_check, done, cold[3];
+    int next_check, done, bad, cold[3];
 };
+__device__ __forceinline__ bool finite_sum(double v) { return v < (double)INFINITY; }   // v >= 0 or NaN
 
 // The first residual and right-hand side (loc: this thread's squares, three
 // components each) against the tolerance: the iterations needed, and the
-// components whose start is worse than zero and is dropped.  One grid barrier.
+// components whose start is worse than zero, or not finite, and is dropped.
+// Every comparison is written so that a NaN does not meet it.  One grid barrier.
 template <typename T>
 __device__ void first_check(const Cheb3Args<T> &a, const double (&loc)[6], int nb, double *sh, Checks &S) {
     double out[6];
@@ -178,7 +182,7 @@ __device__ void first_check(const Cheb3Args<T> &a, const double (&loc)[6], int n
     if (threadIdx.x < 32) {
         // one lane per component
         const int c = threadIdx.x;
-        int need = 0;
+        int need = 0, bad = 0;
         double v = 0.0, u = 0.0;
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -187,8 +191,9 @@ __device__ void first_check(const Cheb3Args<T> &a, const double (&loc)[6], int n
         }
         if (c < 3) {
             const double tol = fmax(a.rtol * sqrt(u), a.atol);
-            S.cold[c] = v > u;
-            v = fmin(v, u);
+            S.cold[c] = !(v <= u);
+            if (!(v <= u)) v = u;
+            bad = !finite_sum(u);
             S.rr[c] = v;
             S.bb[c] = u;
             S.tol2[c] = tol * tol;
@@ -196,13 +201,15 @@ __device__ void first_check(const Cheb3Args<T> &a, const double (&loc)[6], int n
             // iterations more: the error of the slowest modes, which CG
             // damps below its residual, is then below CG's too (16^3 to
             // 31^3, CG1 runs: phi within 2e-11 of a 64-bit run, CG 1.1e-10)
-            if (v > tol * tol) need = iterations_left(v, tol * tol, 3.5f);
+            if (!(v <= tol * tol)) need = iterations_left(v, tol * tol, 3.5f);
         }
         need = max(need, __shfl_down_sync(0xffffffffu, need, 2));
         need = max(need, __shfl_down_sync(0xffffffffu, need, 1));
+        bad = __any_sync(0xffffffffu, bad);
         if (c == 0) {
             S.next_check = min(need, a.max_iter);
-            S.done = need == 0;
+            S.done = need == 0 && !bad;
+            S.bad = bad;
         }
     }
     __syncthreads();
@@ -217,7 +224,8 @@ __device__ void later_check(const Cheb3Args<T> &a, const double *part, int nb, i
         int need = 0;
         for (int c = 0; c < 3; ++c) {
             S.rr[c] = out[c];
-            if (S.rr[c] > S.tol2[c]) need = max(need, iterations_left(S.rr[c], S.tol2[c], 0.0f));
+            if (!finite_sum(out[c])) S.bad = 1;
+            if (!(out[c] <= S.tol2[c])) need = max(need, iterations_left(out[c], S.tol2[c], 0.0f));
         }
         S.done = need == 0;
         S.next_check = min(it + need, a.max_iter);
@@ -279,7 +287,7 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
         }
     }
     int it = 0;
-    while (!S.done && it < a.max_iter) {
+    while (!S.done && !S.bad && it < a.max_iter) {
         ++it;
         const bool check = it == S.next_check;
         const T c1 = a.c1[min(it, kCheb) - 1], c2 = a.c2[min(it, kCheb) - 1];
@@ -312,9 +320,14 @@ __global__ void __launch_bounds__(512, 2) k_mass_cheb3(const __grid_constant__ C
         grid.sync();
         if (check) later_check(a, part, nb, it, S);
     }
+    // not finite: a field that shows it, and zero as the next start
     for (int i = gtid; i < n; i += gs) {
         const V3<T> x = load3(a.x, i);
-        const double ex = (double)x.x + a.e0[0], ey = (double)x.y + a.e0[1], ez = (double)x.z + a.e0[2];
+        double ex = (double)x.x + a.e0[0], ey = (double)x.y + a.e0[1], ez = (double)x.z + a.e0[2];
+        if (S.bad) {
+            store3(a.x, i, V3<T>{0, 0, 0});
+            ex = ey = ez = nan("");
+        }
         if (a.ev) {
             reinterpret_cast<double2 *>(a.ev)[2 * (size_t)i] = make_double2(ex, ey);
             reinterpret_cast<double2 *>(a.ev)[2 * (size_t)i + 1] = make_double2(ez, 0.0);
@@ -453,7 +466,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) k_mass_cheb3_reg(const __grid_
         grid.sync();
     }
     int it = 0;
-    while (!S.done && it < a.max_iter) {
+    while (!S.done && !S.bad && it < a.max_iter) {
         ++it;
         const bool check = it == S.next_check;
         const T c1 = a.c1[min(it, kCheb) - 1], f = a.c2[min(it, kCheb) - 1] * dinv;
@@ -489,8 +502,8 @@ __global__ void __launch_bounds__(kRegThreads, 1) k_mass_cheb3_reg(const __grid_
         for (int q = 0; q < NC; ++q) {
             const int cq = NC == 1 ? comp : q;
             const size_t o = 4 * (size_t)i + cq;
-            const double v = (double)x[q] + a.e0[cq];
-            a.x[o] = x[q];
+            const double v = S.bad ? nan("") : (double)x[q] + a.e0[cq];
+            a.x[o] = S.bad ? (T)0 : x[q];
             if (a.ev) a.ev[o] = v;
             if (a.evf) a.evf[o] = (float)v;
             if (cq == 2) {
