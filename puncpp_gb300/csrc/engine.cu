@@ -2605,6 +2605,10 @@ int pg_run_steps(pg_sim *s, const pg_step_args *a, pg_object *objects, int32_t n
     int32_t oi[2];
     PG_CUDA(cudaMemcpy(oi, s->pcg_out_i, sizeof(oi), cudaMemcpyDeviceToHost));
     if (oi[1] != 0) return fail(PG_ERR_NOT_CONVERGED, "pg_run_steps: the last PCG solve did not converge");
+    if (a->efield_cg1) {
+        PG_CUDA(cudaMemcpy(oi, s->es_out_i, sizeof(oi), cudaMemcpyDeviceToHost));
+        if (oi[1] != 0) return fail(PG_ERR_NOT_CONVERGED, "pg_run_steps: the last ESolver solve did not converge");
+    }
     return PG_OK;
 }
 
