@@ -136,10 +136,10 @@ __global__ void __launch_bounds__(512, 2) k_mixed(DevMesh m, DevParticles p, int
             if (MOVE) {
                 x = fmaf(mp.dt, vx, x); y = fmaf(mp.dt, vy, y); z = fmaf(mp.dt, vz, z);
                 if (PERIODIC) {
-                    // 0 < x < L: the floor is 0
-                    if (!(x > 0.0f && x < mp.Ld[0])) x -= mp.Ld[0] * floorf(x / mp.Ld[0]);
-                    if (!(y > 0.0f && y < mp.Ld[1])) y -= mp.Ld[1] * floorf(y / mp.Ld[1]);
-                    if (!(z > 0.0f && z < mp.Ld[2])) z -= mp.Ld[2] * floorf(z / mp.Ld[2]);
+                    // 0 < x < L, L finite: the floor is 0
+                    if (!(x > 0.0f && x < mp.Ld[0] && mp.Ld[0] < INFINITY)) x -= mp.Ld[0] * floorf(x / mp.Ld[0]);
+                    if (!(y > 0.0f && y < mp.Ld[1] && mp.Ld[1] < INFINITY)) y -= mp.Ld[1] * floorf(y / mp.Ld[1]);
+                    if (!(z > 0.0f && z < mp.Ld[2] && mp.Ld[2] < INFINITY)) z -= mp.Ld[2] * floorf(z / mp.Ld[2]);
                 }
                 p.xf[i] = x; p.yf[i] = y; p.zf[i] = z;
             }

@@ -170,11 +170,14 @@ __device__ __forceinline__ int walk_fp64(const DevMesh &m, double x, double y, d
 // -L <= x <= -1e-200 the rounded quotient stays on its side of the integers
 // (it has a neighbour of the integer between), so the results are the same
 // bits.  The first test, the common one, is an integer comparison (positive
-// doubles order as their bits).  L must lie in (0, 1e100].
+// doubles order as their bits).  For L outside (0, 1e100] (negative, zero, not
+// finite) the formula stands as it is; L is the same for all particles, so its
+// test costs an integer comparison.
 __device__ __forceinline__ double wrap_periodic(double x, double L) {
     const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
-    if (bx - 1 < (unsigned long long)__double_as_longlong(L) - 1) return x;
-    if (L > 0.0 && L <= 1e100) {
+    const unsigned long long bl = (unsigned long long)__double_as_longlong(L);
+    if (bl - 1 < (unsigned long long)__double_as_longlong(1e100)) {
+        if (bx - 1 < bl - 1) return x;
         if (x >= L && x < 2.0 * L) return __dadd_rn(x, -L);
         if (x <= -1e-200 && x >= -L) return __dadd_rn(x, L);
     }
