@@ -1146,6 +1146,7 @@ int pg_create(const pg_mesh *mesh, const pg_config *cfg_in, pg_sim **out) {
             X = std::max(X, std::max(std::fabs(h.bbox_lo[j]), std::fabs(h.bbox_hi[j])) + h.bbox_hi[j] - h.bbox_lo[j]);
         launch_float_tables(d_bary, d_planes, reinterpret_cast<const int4 *>(d_nbr), (int32_t)h.nc, 4.0 * X, cf, d_abs,
                             s->stream);
+        s->dm.lam_inv_range = (float)(1.0 / (4.0 * X));
         if (cudaMemcpyAsync(&s->dm.lam_abs, d_abs, sizeof(float), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
             cudaStreamSynchronize(s->stream) != cudaSuccess)
             return bail(fail(PG_ERR_CUDA, "pg_create: cell records"));

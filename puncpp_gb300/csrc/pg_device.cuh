@@ -51,9 +51,10 @@ struct DevMesh {
     // mixed form's deposit and field read, in one aligned pair of sectors
     const float4 *cell_f = nullptr;   // [nc][4]
     float *E_f = nullptr;             // [nc][4] FP32 field (mixed form)
-    // bound on the rounding of the FP64 tables in lambda (launch_float_tables),
-    // for points within lam_range of the origin in every coordinate
-    float lam_abs = 0.0f;
+    // bound on the rounding of the FP64 tables in lambda (launch_float_tables)
+    // for points with coordinates up to 1 / lam_inv_range; beyond, it grows with
+    // the largest coordinate (point_bound)
+    float lam_abs = 0.0f, lam_inv_range = 0.0f;
     // CG1 (vertex) field of the ESolver path: [ndof][4] (x, y, z, 0)
     const double *Ev = nullptr;
     const float *Evf = nullptr;
