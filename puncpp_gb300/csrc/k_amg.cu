@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "pg_device.cuh"
@@ -899,29 +900,37 @@ int pcg_amg_grid_blocks() {
     return g;
 }
 
-// Largest cluster (a power of two) that this device runs with the kernel.
-static int cluster_blocks() {
-    static int g = 0;
-    if (g == 0) {
-        const void *fn = (const void *)k_pcg_amg<ClusterSync, 2>;
-        int best = 1;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
-        for (int k = kClusterMax; k > 1; k /= 2) {
-            cudaLaunchConfig_t cfg{};
-            cudaLaunchAttribute at{};
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = k;
-            at.val.clusterDim.y = at.val.clusterDim.z = 1;
-            cfg.gridDim = dim3(k);
-            cfg.blockDim = dim3(kPcgThreads);
-            cfg.attrs = &at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) { best = k; break; }
-            cudaGetLastError();
-        }
-        g = best;
+// Largest cluster (a power of two) of the kernel on the current device.
+static int query_cluster_blocks() {
+    const void *fn = (const void *)k_pcg_amg<ClusterSync, 2>;
+    const bool large = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (!large) cudaGetLastError();
+    for (int k = large ? kClusterMax : 8; k > 1; k /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = k;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(k);
+        cfg.blockDim = dim3(kPcgThreads);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) return k;
+        cudaGetLastError();
     }
+    return 1;
+}
+
+// Found once per device: a kernel's attributes are the device's, so the size
+// that one device takes says nothing about another in the same process.
+static int cluster_blocks() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];   // 0: not yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return query_cluster_blocks();
+    int g = known[dev].load(std::memory_order_relaxed);
+    if (g == 0) known[dev].store(g = query_cluster_blocks(), std::memory_order_relaxed);
     return g;
 }
 
