@@ -1,13 +1,13 @@
 // PCG preconditioned by one smoothed-aggregation AMG V-cycle per iteration,
 // all in one launch (a cooperative grid, or one thread-block cluster).
 //
-// Krylov recurrence in FP32 with the solution and the true-residual
-// replacements in FP64, inner products of FP32 values summed in double-float
-// (48 bits) across threads, FP32 step lengths; the stopping test is on the FP64
-// true residual ||b - A x|| <= max(rtol ||b||, atol).  A replacement before
-// the end of a solve (hierarchies of three or more levels) takes the true
-// residual inside the iteration's own V-cycle; the one at the end is a new
-// pass that restarts the cycle from the true residual.
+// Krylov recurrence in FP32 with the solution, the inner products, the step
+// lengths and the true-residual replacements in FP64 (p.Ap and the
+// recurrence's ||r||^2 from one FP32 sum per thread, r.z from FP64 products);
+// the stopping test is on the FP64 true residual ||b - A x|| <= max(rtol ||b||,
+// atol).  A replacement before the end of a solve (hierarchies of three or more
+// levels) takes the true residual inside the iteration's own V-cycle; the one
+// at the end is a new pass that restarts the cycle from the true residual.
 //
 // The V-cycle (one weighted-Jacobi sweep from zero before the coarse
 // correction and one after, Galerkin coarse operators, dense coarsest
@@ -17,10 +17,10 @@
 // with the last restriction and the coarse solve in one product
 // (G = C^-1 S^T) and the up-sweep of levels >= 1 collapsed into one product
 // (U1 = [S_1 | S_1 S_2 | ...]).  For L >= 2 levels above the coarsest an
-// iteration is L + 3 grid phases:
-//   A p = A z + beta A p_old and the sums that give alpha;
-//   x, r, s = w D^-1 r of the step, and b_1 -= alpha S_0^T A p (the restriction
-//     of the new residual from that of the old one: one gather per entry);
+// iteration is L + 4 grid phases:
+//   A p = A z + beta A p_old and the sum that gives alpha;
+//   x, r, s = w D^-1 r of the step, and ||r||^2;
+//   b_1 = S_0^T r;
 //   per level 1 .. L-1: the restriction (at L-1: G) and the smoothing W_l b_l
 //     on disjoint blocks;
 //   y_1 = t_1 + U1 [t_2 .. t_{L-1}, y_L];
@@ -30,10 +30,12 @@
 //
 // What bounds it: the chain of dependent loads of each phase (entries, then
 // gathers) and the barriers; at 80^3 also the L2, at 4 to 4.5 TB/s in the two
-// phases that stream the level-0 operators.  Solves (GB300), before this form ->
-// with it -> with the cluster form, sums without divergent shuffles, spread rows
-// and operands loaded ahead: 80^3 probe (531k rows) 1.63 -> 1.28 -> 1.21 ms, 56^3
-// (185k) 1.10 -> 0.79 -> 0.74, 16^3 periodic (4096) 0.69 -> 0.43 -> 0.28.
+// phases that stream the level-0 operators.  Solves (GB300): 80^3 probe (531k
+// rows) 1.18 ms, 56^3 (185k) 0.75, 40^3 (68,908) 0.43, 16^3 periodic (4,096)
+// 0.29.  With double-float sums, FP32 step lengths and b_1 updated from step to
+// step (b_1 -= alpha S_0^T A p, a phase less) it was 1.20, 0.74, 0.37 and 0.28 ms,
+// but with 48 bits where the sums have 53 and a b_1 that drifts from r.  The
+// figures at Span and the launch, unless dated, compare two forms with those sums.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -63,27 +65,6 @@ namespace {
 // slower at 185k rows).  Arrays of a conditional load are zeroed: left
 // undefined, the compiler carried them around the whole loop and spilled.
 
-// Double-float sums (unevaluated hi + lo, 48 bits) of FP32 values: exact
-// two-operand sums (Knuth) and products by the fused residual.  One warp-wide
-// FP64 add occupies a sub-partition for 64 cycles; these use the FP32 pipe.
-struct __align__(8) DF {   // moved as one 8-byte value
-    float hi, lo;
-};
-__device__ __forceinline__ DF df_add(DF a, DF b) {
-    const float s = __fadd_rn(a.hi, b.hi), t = __fsub_rn(s, a.hi);
-    const float e = __fadd_rn(__fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, t)), __fsub_rn(b.hi, t)), __fadd_rn(a.lo, b.lo));
-    const float h = __fadd_rn(s, e);
-    return DF{h, __fsub_rn(e, __fsub_rn(h, s))};
-}
-__device__ __forceinline__ DF df_fma(float x, float y, DF a) {
-    const float p = __fmul_rn(x, y);
-    return df_add(a, DF{p, fmaf(x, y, -p)});
-}
-__device__ __forceinline__ DF df_mul(DF a, float b) {
-    const float p = __fmul_rn(a.hi, b);
-    return df_add(DF{p, fmaf(a.hi, b, -p)}, DF{__fmul_rn(a.lo, b), 0.0f});
-}
-
 constexpr int kWarps = kPcgThreads / 32;
 
 // The barrier between phases: of a cooperative grid, or of one thread-block
@@ -102,70 +83,91 @@ struct ClusterSync {
 constexpr int kClusterMax = 16;   // blocks of a cluster
 
 // Store v at this shared-memory address of block `rank` of the cluster.
-__device__ __forceinline__ void store_remote(DF *p, DF v, int rank) {
+__device__ __forceinline__ void store_remote(double *p, double v, int rank) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    asm volatile("{\n\t.reg .b32 q;\n\tmapa.shared::cluster.u32 q, %0, %1;\n\tst.shared::cluster.v2.f32 [q], {%2, %3};\n\t}"
-                 ::"r"(a), "r"(rank), "f"(v.hi), "f"(v.lo)
+    asm volatile("{\n\t.reg .b32 q;\n\tmapa.shared::cluster.u32 q, %0, %1;\n\tst.shared::cluster.f64 [q], %2;\n\t}"
+                 ::"r"(a), "r"(rank), "d"(v)
                  : "memory");
 }
 
-// Sums of K values over the block, for grid_total after the caller's barrier:
-// one thread's store to part[q * nb + blockIdx.x] in global memory, or in a
-// cluster to part[q * kClusterMax + blockIdx.x] in every block's shared memory
-// (read there without a trip to the L2).  sh: kWarps * K values.
-//
-// Every warp runs the shuffles of both functions, though K of them suffice: a
-// shuffle where the warp may have diverged (under a test of the warp's number,
-// or after loads by a part of the lanes) took 250 cycles instead of 25, and a
-// total 1.3 us (cluster) to 2.6 (77 blocks) instead of 0.3 to 0.8.
-template <int K, class Sync>
-__device__ __forceinline__ void block_part(DF (&v)[K], DF *sh, DF *part, int nb) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < K; ++q) {
-        for (int o = 16; o > 0; o >>= 1)
-            v[q] = df_add(v[q], DF{__shfl_down_sync(0xffffffffu, v[q].hi, o), __shfl_down_sync(0xffffffffu, v[q].lo, o)});
-        if (lane == 0) sh[q * kWarps + w] = v[q];
-    }
+// Inner products are summed in FP64.  A warp-wide FP64 add takes a
+// sub-partition of an SM 64 cycles, so the sums go through shared memory in
+// steps that keep each addition on one warp of every sub-partition: the 512
+// threads' values in four by warps 0-3, the 128 sums in four by warp 0, and its
+// five rounds of shuffles (1,340 cycles with its barriers; 2,240 with every
+// warp's own five rounds first, 1,980 with the rounds in four warps).
+template <int N = 32>   // the sum of each N lanes
+__device__ __forceinline__ double warp_sum(double v) {
+    for (int o = N / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ double sum4(const double *p, int step) { return (p[0] + p[step]) + (p[2 * step] + p[3 * step]); }
+
+// The block's sum of v, for the total after the caller's barrier: stored to
+// part[blockIdx.x] in global memory, or in a cluster in every block's shared
+// memory (read there without a trip to the L2).  sh: 1.25 kPcgThreads values.
+template <class Sync, class T>
+__device__ __forceinline__ void block_part(T v, double *sh, double *part, int nb) {
+    const int t = threadIdx.x, q = kPcgThreads / 4;
+    T *f = reinterpret_cast<T *>(sh);
+    double *s = sh + kPcgThreads;
+    f[t] = v;
     __syncthreads();
-    DF s = sh[(w < K ? w : 0) * kWarps + (lane & (kWarps - 1))];
-    for (int o = kWarps / 2; o > 0; o >>= 1)
-        s = df_add(s, DF{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
-    if (Sync::kCluster) {
-        if (w < K && lane < nb) store_remote(part + w * kClusterMax + blockIdx.x, s, lane);
-    } else {
-        if (w < K && lane == 0) part[w * nb + blockIdx.x] = s;
+    if (t < q) s[t] = ((double)f[t] + (double)f[t + q]) + ((double)f[t + 2 * q] + (double)f[t + 3 * q]);
+    __syncthreads();
+    if (t < 32) {
+        const double a = warp_sum(sum4(s + t, 32));
+        if (Sync::kCluster) {
+            if (t < nb) store_remote(part + blockIdx.x, a, t);
+        } else if (t == 0) {
+            part[blockIdx.x] = a;
+        }
     }
 }
 
-// Totals of the K partial sums over the blocks (the same order in every
-// block: the same totals) in tot[0..K); valid after the call.
-template <int K, class Sync>
-__device__ __forceinline__ void grid_total(const DF *part, int nb, DF *tot) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    DF s{0.0f, 0.0f};
+// Total of the blocks' sums (the same order in every block: the same total),
+// by one warp.  Its lanes meet first and all of them load, some in vain: in a
+// warp that counts as diverged (after a barrier that one lane spins in, after
+// loads by a part of the lanes) a shuffle takes 250 cycles and not 25.
+template <class Sync>
+__device__ __forceinline__ double warp_total(const double *part, int nb) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
     if (Sync::kCluster) {
         const int b = lane & (kClusterMax - 1);
-        const DF v = part[(w < K ? w : 0) * kClusterMax + b];
-        s = DF{b < nb ? v.hi : 0.0f, b < nb ? v.lo : 0.0f};
-    } else {
-        const float2 *p = reinterpret_cast<const float2 *>(part + (w < K ? w : 0) * nb);
-        for (int k = 0; k < nb; k += 5 * 32) {
-            float2 v[5];
-#pragma unroll
-            for (int u = 0; u < 5; ++u) {
-                const int i = k + 32 * u + lane;
-                v[u] = make_float2(0.0f, 0.0f);
-                if (w < K && i < nb) v[u] = __ldcg(p + i);
-            }
-#pragma unroll
-            for (int u = 0; u < 5; ++u) s = df_add(s, DF{v[u].x, v[u].y});
-        }
+        const double v = part[b];
+        return warp_sum<kClusterMax>(b < nb ? v : 0.0);
     }
-    for (int o = Sync::kCluster ? kClusterMax / 2 : 16; o > 0; o >>= 1)
-        s = df_add(s, DF{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
-    if (w < K && lane == 0) tot[w] = s;
+    double a = 0.0;
+    for (int k = 0; k < nb; k += 5 * 32) {
+        double v[5];
+#pragma unroll
+        for (int u = 0; u < 5; ++u) {
+            const int i = k + 32 * u + lane;
+            const double p = __ldcg(part + (i < nb ? i : 0));
+            v[u] = i < nb ? p : 0.0;
+        }
+        a += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+    }
+    return warp_sum(a);
+}
+// The same in warp 0, by warps 0-3 of a grid's block; every thread of the block
+// calls it.
+template <class Sync>
+__device__ __forceinline__ double block_total(const double *part, int nb, double *sh) {
+    if (Sync::kCluster) return threadIdx.x < 32 ? warp_total<Sync>(part, nb) : 0.0;
+    const int t = threadIdx.x, q = kPcgThreads / 4;
+    if (t < q) {
+        double a = 0.0;
+        for (int k = t; k < nb; k += 3 * q) {
+            const double v0 = __ldcg(part + k), v1 = k + q < nb ? __ldcg(part + k + q) : 0.0;
+            const double v2 = k + 2 * q < nb ? __ldcg(part + k + 2 * q) : 0.0;
+            a += (v0 + v1) + v2;
+        }
+        sh[t] = a;
+    }
     __syncthreads();
+    return t < 32 ? warp_sum(sum4(sh + t, 32)) : 0.0;
 }
 
 // ---- the work of a block ------------------------------------------------------
@@ -418,20 +420,16 @@ __device__ __forceinline__ void product(const SpOp &S, const float *x, E &e, Spa
 }
 
 // ---- what a product's rows become -------------------------------------------
-// b = S^T x (keep 0) or b - alpha S^T x (keep 1: x = A p, the restriction of
-// the CG step's residual from that of the last one), and sb = omega D^-1 b
-// for the level's smoother (sb null: none).
+// b = S^T x and sb = omega D^-1 b for the level's smoother (sb null: none).
 struct RestrictRow {
-    struct Pre { float b, d; };
+    using Pre = float;
     float *b, *sb;
     const float *dinv;
-    float om, alpha;
-    bool update;
-    __device__ __forceinline__ Pre pre(int i) const { return Pre{update ? b[i] : 0.0f, sb ? __ldg(dinv + i) : 0.0f}; }
-    __device__ __forceinline__ void row(int i, float s, const Pre &p) const {
-        const float v = update ? fmaf(-alpha, s, p.b) : s;
-        b[i] = v;
-        if (sb) sb[i] = om * p.d * v;
+    float om;
+    __device__ __forceinline__ Pre pre(int i) const { return sb ? __ldg(dinv + i) : 0.0f; }
+    __device__ __forceinline__ void row(int i, float s, Pre d) const {
+        b[i] = s;
+        if (sb) sb[i] = om * d * s;
     }
 };
 // t = W x = omega D^-1 (2 x - A omega D^-1 x) from sx = omega D^-1 x.
@@ -455,11 +453,11 @@ struct DirectRow {
     using Pre = float;
     float *z;
     const float *r;
-    DF rz;
+    double rz;
     __device__ __forceinline__ Pre pre(int i) const { return r[i]; }
     __device__ __forceinline__ void row(int i, float s, Pre ri) {
         z[i] = s;
-        rz = df_fma(s, ri, rz);
+        rz = fma((double)s, (double)ri, rz);
     }
 };
 
@@ -493,9 +491,9 @@ struct Prolong {
             sell_load(S, hs.off(i0), hs.width(), es);
         }
     }
-    __device__ __forceinline__ DF rows(const SpOp &A, const SpOp &S, const float *s, const float *y, const float *r,
-                                       const float *dinv, float om, float *z, int i0, int i1, int st) {
-        DF rz{0.0f, 0.0f};
+    __device__ __forceinline__ double rows(const SpOp &A, const SpOp &S, const float *s, const float *y, const float *r,
+                                           const float *dinv, float om, float *z, int i0, int i1, int st) {
+        double rz = 0.0;
         if (!kAhead) {
             ha.load(A, i0, i1);
             hs.load(S, i0, i1);
@@ -511,14 +509,14 @@ struct Prolong {
             const float u = sell_sum(S, y, os, ws, cs, es);
             const float v = fmaf(-om * di, q, (2.0f - om) * si) + u;
             z[i] = v;
-            rz = df_fma(v, ri, rz);
+            rz = fma((double)v, (double)ri, rz);
         }
         return rz;
     }
 };
 
-// p = z + beta p, Ap = A z + beta Ap (none: the
-// first step, no reads of p and Ap), and this thread's shares of p.Ap, r.Ap and Ap.Ap.
+// p = z + beta p, Ap = A z + beta Ap (none: the first step, no reads of p and
+// Ap), and this thread's share of p.Ap in FP32.
 template <bool kAhead>
 struct Direction {
     SellHead h;
@@ -533,27 +531,23 @@ struct Direction {
         h.load(A, i0, i1);
         if (i0 < i1) load(A, diag, i0);
     }
-    __device__ __forceinline__ void rows(const SpOp &A, const float *diag, const float *z, const float *r, float *p,
-                                         float *Ap, float beta, bool none, DF (&v)[3], int i0, int i1, int st) {
-        float pap = 0.0f, rap = 0.0f, apap = 0.0f;
+    __device__ __forceinline__ float rows(const SpOp &A, const float *diag, const float *z, float *p, float *Ap,
+                                          float beta, bool none, int i0, int i1, int st) {
+        float pap = 0.0f;
         if (!kAhead) h.load(A, i0, i1);
         for (int i = i0; i < i1; i += st) {
             if (!kAhead || i != i0) load(A, diag, i);
             const int off = h.off(i), w = h.width(), cb = h.h.y;
             h.load(A, i + st, i1);
-            const float zi = z[i], ri = r[i];
+            const float zi = z[i];
             const float p0 = none ? 0.0f : p[i], q0 = none ? 0.0f : Ap[i];
             const float s = fmaf(di, zi, a0_sum(A, z, off, w, cb, e));
             const float pi = fmaf(beta, p0, zi), api = fmaf(beta, q0, s);
             p[i] = pi;
             Ap[i] = api;
             pap = fmaf(pi, api, pap);
-            rap = fmaf(ri, api, rap);
-            apap = fmaf(api, api, apap);
         }
-        v[0] = DF{pap, 0.0f};
-        v[1] = DF{rap, 0.0f};
-        v[2] = DF{apap, 0.0f};
+        return pap;
     }
 };
 
@@ -590,15 +584,8 @@ __device__ __forceinline__ double true_residual(const PcgArgs &a, float *r, floa
     return rr;
 }
 
-// The level-0 restriction, at three places of the loop: one copy.
-__device__ __noinline__ void restrict0(const SpOp &S, const float *x, float *b, float *sb, const float *dinv, float om,
-                                       float alpha, bool update, Span sp) {
-    RestrictRow e{b, sb, dinv, om, alpha, update};
-    product<true>(S, x, e, sp);
-}
-
-// x += alpha p, r -= alpha Ap, s = omega D^-1 r of this thread's rows.  The
-// operands of its first rows (p and Ap written by the same thread) are loaded
+// x += alpha p, r -= alpha Ap, s = omega D^-1 r of this thread's rows, and its
+// share of the new ||r||^2 in FP32.  The operands of its first rows (p and Ap written by the same thread) are loaded
 // before the barrier and the sums that give alpha.
 struct CgUpdate {
     static constexpr int R = 4;
@@ -616,42 +603,52 @@ struct CgUpdate {
             d[k] = ok ? __ldg(a.dinv32 + j) : 0.0f;
         }
     }
-    __device__ __forceinline__ void apply(const PcgArgs &a, float *s, float om, float alpha, int i, int i1, int gst) const {
+    __device__ __forceinline__ float apply(const PcgArgs &a, float *s, float om, double alpha, int i, int i1, int gst,
+                                           float rr) const {
+        const float alpha32 = (float)alpha;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int j = i + k * gst;
             if (j < i1) {
-                const float n = fmaf(-alpha, q[k], r[k]);
-                a.x[j] = fma((double)alpha, (double)p[k], x[k]);
+                const float n = fmaf(-alpha32, q[k], r[k]);
+                a.x[j] = fma(alpha, (double)p[k], x[k]);
                 a.r32[j] = n;
                 s[j] = om * d[k] * n;
+                rr = fmaf(n, n, rr);
             }
         }
+        return rr;
     }
 };
 
-// Partial sums in a.partials: [0, 3 nb) p.Ap, r.Ap, Ap.Ap; [3 nb, 4 nb) r.z
-// (double-float; a cluster keeps them in shared memory); [4 nb, 6 nb) the FP64 true residual's and right-hand side's
-// squares.  A buffer is written again only after at least one barrier has
-// passed since every block read it.
+// Partial sums: p.Ap in A, r.z in C, ||r||^2 of the recurrence in E (a cluster
+// keeps these in shared memory); the FP64 true residual's and the right-hand
+// side's squares in B and D.  A buffer is written again only after at least one
+// barrier has passed since every block read it.
 template <class Sync, int kBlocks>
 __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_constant__ PcgArgs a,
                                                             const __grid_constant__ AmgDev M) {
-    constexpr bool kAhead = kBlocks == 1;
-    __shared__ double sh[2 * kPcgThreads + 16];   // FP64 sums; the double-float ones use its head
-    __shared__ DF tot[3];
-    __shared__ double scal[2];                    // FP64 scalars; 1: go on
-    DF *shf = reinterpret_cast<DF *>(sh);
+    constexpr bool kAhead = kBlocks == 1 && !Sync::kCluster;
+    __shared__ double sh[2 * kPcgThreads + 16];
     const int nb = gridDim.x, n = a.n, L = M.nlev - 1;
     const Span all{(int)blockIdx.x, nb, n <= nb * kPcgThreads};
     const int i0 = all.first(), i1 = n, gst = all.stride();
-    __shared__ DF part_cluster[Sync::kCluster ? 4 * kClusterMax : 1];
-    DF *partA = Sync::kCluster ? part_cluster : reinterpret_cast<DF *>(a.partials);
-    DF *partC = partA + 3 * (Sync::kCluster ? kClusterMax : nb);
-    double *partB = a.partials + 4 * nb, *partD = a.partials + 5 * nb;
+    __shared__ double part_cluster[Sync::kCluster ? 3 * kClusterMax : 1];
+    const int pst = Sync::kCluster ? kClusterMax : nb;
+    double *partA = Sync::kCluster ? part_cluster : a.partials;
+    double *partC = partA + pst, *partE = partA + 2 * pst;
+    double *partB = a.partials + 3 * nb, *partD = a.partials + 4 * nb;
     const float om0 = M.lev[0].omega;
     float *r = a.r32, *z = a.z32, *s0 = M.s0;
     double ra, rb;
+    // solver scalars, kept by warp 0 (no registers held across the loop)
+    __shared__ double t_rz, t_tol2, t_rr, t_bb, t_alpha, t_mean;
+    __shared__ float t_beta;
+    __shared__ int t_status, t_updates, t_pass, t_go;
+    // what the recurrence's ||r||^2 asks for: go on, replace the residual
+    // inside this cycle, start a new pass (the last warp's)
+    enum { kGoOn, kKeep, kNewPass };
+    __shared__ int t_next;
 
     if (a.remove_mean) {
         double s = 0.0;
@@ -660,37 +657,32 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
         if (threadIdx.x == 0) partD[blockIdx.x] = ra;
         Sync::sync();
         grid_sum2(partD, nullptr, nb, sh, ra, rb);
-        if (threadIdx.x == 0) scal[0] = ra / (double)n;
+        if (threadIdx.x == 0) t_mean = ra / (double)n;
         __syncthreads();
-        const double mean = scal[0];
+        const double mean = t_mean;
         for (int i = i0; i < i1; i += gst) a.b[i] = a.b[i] - mean;
         Sync::sync();
     }
-    // Solver scalars, in shared memory (no registers held across the loop).
-    // The step lengths are FP32 (x and r take the same alpha; any alpha near
-    // the minimiser keeps the recurrence consistent) and the recurrence's
-    // ||r||^2 double-float, so every thread forms them from the totals itself:
-    // one thread's chain of FP64 operations, a division among them, was 2 us of
-    // each of an iteration's two scalar steps, its FP32 chain with a barrier
-    // after it 0.5 to 0.8.  FP32 values are compared with the largest FP32
-    // value not above an FP64 bound, which decides as the FP64 comparison.
-    // rz and rec: by the parity of the step, as some threads still read the
-    // last one's.
-    __shared__ double t_tol2, t_rr, t_bb;
-    __shared__ float t_small, t_fell;             // bounds of the recurrence's ||r||^2
-    __shared__ DF t_rec[2], t_rz[2];
-    __shared__ int t_status, t_updates, t_pass;
     if (threadIdx.x == 0) {
-        t_tol2 = t_rr = t_bb = 0.0;
+        t_tol2 = t_rr = t_bb = t_rz = 0.0;
         t_status = 1; t_updates = 0; t_pass = 0;
     }
     int it = 0;                                   // CG steps taken
-    float beta = 0.0f;
+    // the recurrence's ||r||^2 (complete in E) in the last warp, beside the
+    // restriction, of which it has the fewest rows: waited for by all threads it
+    // is 0.8 us of an iteration.  (The warp's number by a shuffle, and t_next
+    // from all its lanes: the warp then counts as converged.)
+    auto look = [&] {
+        if (__shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0) != kWarps - 1) return;
+        const double rec = warp_total<Sync>(partE, nb);
+        const bool last = rec <= t_tol2 || it >= a.max_iter, fell = rec <= 1e-6 * t_rr;
+        t_next = last || (fell && L < 2) ? kNewPass : fell ? kKeep : kGoOn;
+    };
     // fresh: start a pass, from the FP64 true residual; else a CG step
     bool fresh = true;
     Direction<kAhead> dir;
     for (;;) {
-        bool keep = false;
+        int next = kGoOn;
         if (fresh) {
             double bb = 0.0;
             const double rr = true_residual(a, r, s0, om0, it == 0, bb, i0, i1, gst);
@@ -714,64 +706,61 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
                     ++t_updates;
                 }
                 ++t_pass;
-                t_small = __double2float_rd(t_tol2);
-                t_fell = __double2float_rd(1e-6 * t_rr);
-                t_rec[it & 1] = DF{(float)t_rr, 0.0f};
-                if (t_rr <= t_tol2) { t_status = 0; scal[1] = 0.0; }
-                else if (it >= a.max_iter) { t_status = 1; scal[1] = 0.0; }
-                else if (stalled) { t_status = 3; scal[1] = 0.0; }
-                else scal[1] = 1.0;
+                t_go = 0;
+                if (t_rr <= t_tol2) t_status = 0;
+                else if (it >= a.max_iter) t_status = 1;
+                else if (stalled) t_status = 3;
+                else t_go = 1;
             }
             __syncthreads();
-            if (scal[1] == 0.0) break;
-            if (L >= 2) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
+            if (!t_go) break;
         } else {
-            // p = z + beta p, Ap = A z + beta Ap; p.Ap and the terms of
-            // ||r - alpha Ap||^2 = ||r||^2 - 2 alpha r.Ap + alpha^2 Ap.Ap, which
-            // only decides when the residual is replaced
-            DF v[3];
-            dir.rows(M.lev[0].A, M.diag0, z, r, a.p32, a.Ap32, beta, it == 0, v, i0, i1, gst);
+            // p = z + beta p, Ap = A z + beta Ap, p.Ap
+            const float pap32 = dir.rows(M.lev[0].A, M.diag0, z, a.p32, a.Ap32, t_beta, it == 0, i0, i1, gst);
             CgUpdate up;
             up.load(a, i0, i1, gst);
-            block_part<3, Sync>(v, shf, partA, nb);
+            block_part<Sync>(pap32, sh, partA, nb);
             Sync::sync();
-            grid_total<3, Sync>(partA, nb, tot);
-            const float pap = tot[0].hi;
-            DF rec = t_rec[it & 1];
-            const float alpha = t_rz[it & 1].hi / pap;
-            ++it;
-            if (!(pap > 0.0f)) {
-                if (threadIdx.x == 0) t_status = 2;
-                break;
+            const double pap = block_total<Sync>(partA, nb, sh);
+            if (threadIdx.x == 0) {
+                t_go = pap > 0.0;
+                t_alpha = t_rz / pap;
+                if (!(pap > 0.0)) t_status = 2;
             }
-            const DF rap{-2.0f * tot[1].hi, -2.0f * tot[1].lo};
-            rec = df_add(rec, df_mul(df_add(df_mul(tot[2], alpha), rap), alpha));
-            if (threadIdx.x == 0) t_rec[it & 1] = rec;
-            // replacement: at the end (tolerance or cap) by a new pass; between
-            // (the recurrence fell by 1e6 in ||r||^2) inside this cycle when
-            // L >= 2
-            const bool small = rec.hi <= t_small || it >= a.max_iter, fell = rec.hi <= t_fell;
-            up.apply(a, s0, om0, alpha, i0, i1, gst);
+            __syncthreads();
+            ++it;
+            if (!t_go) break;
+            const double alpha = t_alpha;
+            float rr32 = up.apply(a, s0, om0, alpha, i0, i1, gst, 0.0f);
             for (int i = i0 + CgUpdate::R * gst; i < i1; i += CgUpdate::R * gst) {
                 up.load(a, i, i1, gst);
-                up.apply(a, s0, om0, alpha, i, i1, gst);
+                rr32 = up.apply(a, s0, om0, alpha, i, i1, gst, rr32);
             }
-            if (small || (fell && L < 2)) {
-                Sync::sync();
-                fresh = true;
-                continue;
-            }
-            keep = fell;
-            // restriction of the new residual from that of the old one: one
-            // gather per entry (of Ap) instead of two (r - alpha Ap), and r is
-            // updated in place
-            if (L >= 2) restrict0(M.lev[0].ST, a.Ap32, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, alpha, true, all);
+            block_part<Sync>(rr32, sh, partE, nb);
+            Sync::sync();
+            look();
         }
-        Sync::sync();
         // z = B r
+        if (L >= 2) {
+            // b_1 = S_0^T r: a phase of its own after the update, which gathers one
+            // vector; within the update's phase it would gather r and A p (80^3:
+            // 15 us an iteration more)
+            const AmgLevelDev &V = M.lev[1];
+            RestrictRow e{V.b, V.sb, V.dinv, V.omega};
+            product<true>(M.lev[0].ST, r, e, all);
+        }
+        if (!fresh) {
+            __syncthreads();
+            next = t_next;
+        }
+        if (L >= 2 || next == kNewPass) Sync::sync();
+        if (next == kNewPass) {
+            fresh = true;
+            continue;
+        }
         const float *yup = M.yL;
         if (L == 1) {
-            RestrictRow e{M.yL, nullptr, nullptr, 0.0f, 0.0f, false};
+            RestrictRow e{M.yL, nullptr, nullptr, 0.0f};
             product<false>(M.G, r, e, all);
             Sync::sync();
         }
@@ -788,7 +777,7 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
             }
             if (my != 1) {
                 const AmgLevelDev &N = M.lev[coarse ? l : l + 1];
-                RestrictRow e{coarse ? M.yL : N.b, coarse ? nullptr : N.sb, N.dinv, N.omega, 0.0f, false};
+                RestrictRow e{coarse ? M.yL : N.b, coarse ? nullptr : N.sb, N.dinv, N.omega};
                 if (coarse) product<false>(M.G, V.b, e, sp);
                 else product<true>(V.ST, V.b, e, sp);
             }
@@ -796,7 +785,7 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
                 SmoothRow w{V.t, V.sb, V.dinv, V.omega};
                 product<true>(V.A, V.sb, w, sp);
             }
-            if (keep && coarse) {
+            if (next == kKeep && coarse) {
                 // replacement inside the cycle: the FP64 true residual of x
                 // (complete here) into r; z = B r of the recurrence's r stands
                 // for B of the true one (they differ by the recurrence's drift)
@@ -807,50 +796,52 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
             }
             Sync::sync();
         }
-        DF v[1];
+        double rz;
         if (L >= 1) {
             const SpOp &A0 = M.lev[0].A;
             if (L >= 2) {
                 AddRow e{M.y1, M.lev[1].t};
                 product<true>(M.U1, M.stack, e, all);
-                if (keep) restrict0(M.lev[0].ST, r, M.lev[1].b, M.lev[1].sb, M.lev[1].dinv, M.lev[1].omega, 0.0f, false, all);
                 yup = M.y1;
             }
             auto up = [&](auto pro) {
                 pro.first(A0, M.S0, s0, r, a.dinv32, i0, i1);
                 if (L >= 2) Sync::sync();
-                v[0] = pro.rows(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
+                rz = pro.rows(A0, M.S0, s0, yup, r, a.dinv32, om0, z, i0, i1, gst);
             };
             if (M.S0.c16) up(Prolong<FmtH16, kAhead>{});
             else up(Prolong<FmtH32, kAhead>{});
         } else {
-            DirectRow e{z, r, DF{0.0f, 0.0f}};
+            DirectRow e{z, r, 0.0};
             product<false>(M.cinv, r, e, all);
-            v[0] = e.rz;
+            rz = e.rz;
         }
         dir.first(M.lev[0].A, M.diag0, i0, i1);
-        block_part<1, Sync>(v, shf, partC, nb);
+        block_part<Sync>(rz, sh, partC, nb);
         Sync::sync();
-        grid_total<1, Sync>(partC, nb, t_rz + (it & 1));
-        if (keep) {
+        rz = block_total<Sync>(partC, nb, sh);
+        if (threadIdx.x == 0) {
+            // the direction continues across replacements
+            t_beta = it == 0 ? 0.0f : (float)(rz / t_rz);
+            t_rz = rz;
+        }
+        if (next == kKeep) {
             // the true residual replaces the recurrence's (as at a pass start,
             // with the same stall test)
             grid_sum2(partD, nullptr, nb, sh, ra, rb);
             if (threadIdx.x == 0) {
                 const bool stalled = ra > 1e-2 * t_rr;
                 t_rr = ra;
-                t_fell = __double2float_rd(1e-6 * t_rr);
-                t_rec[it & 1] = DF{(float)ra, 0.0f};
                 ++t_updates;
-                scal[1] = 1.0;
-                if (t_rr <= t_tol2) { t_status = 0; scal[1] = 0.0; }
-                else if (stalled) { t_status = 3; scal[1] = 0.0; }
+                t_go = 0;
+                if (t_rr <= t_tol2) t_status = 0;
+                else if (stalled) t_status = 3;
+                else t_go = 1;
             }
             __syncthreads();
-            if (scal[1] == 0.0) break;
+            if (!t_go) break;
         }
-        // the direction continues across replacements
-        beta = it == 0 ? 0.0f : t_rz[it & 1].hi / t_rz[(it & 1) ^ 1].hi;
+        __syncthreads();
         fresh = false;
     }
     if (a.remove_mean) {
@@ -861,9 +852,9 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
         if (threadIdx.x == 0) partB[blockIdx.x] = ra;
         Sync::sync();
         grid_sum2(partB, nullptr, nb, sh, ra, rb);
-        if (threadIdx.x == 0) scal[0] = ra / (double)n;
+        if (threadIdx.x == 0) t_mean = ra / (double)n;
         __syncthreads();
-        const double mean = scal[0];
+        const double mean = t_mean;
         for (int i = i0; i < i1; i += gst) a.x[i] = a.x[i] - mean;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -879,12 +870,14 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
 
 // Systems of at most kClusterRows rows run on one cluster, as many blocks (a
 // power of two, at most 16) as leave kClusterRowsPerBlock rows to each: its
-// barrier is the hardware's (0.3 against 1.3 us of a cooperative grid, five
+// barrier is the hardware's (0.3 against 1.3 us of a cooperative grid, six
 // times an iteration) and its sums stay in shared memory, while its 16 SMs are
 // enough for so few rows.  Measured, solve on the grid -> on the cluster: 2,744
 // rows 0.84 -> 0.45 ms, 9,260 0.49 -> 0.385, 13,824 0.467 -> 0.474 and, periodic, 0.64
 // -> 0.66, 39,298 0.61 -> 0.93, so the line lies between the second and the
-// third.  Rows per block: 1,000 rows 0.50 / 0.38 / 0.33 / 0.29 ms with 512 / 256 /
+// third.  (With FP64 sums and the restriction in a phase of its own: 9,248 rows
+// 0.437 -> 0.354, 15,606 0.466 -> 0.426, 24,362 0.462 -> 0.515; the line could lie at
+// 17,000 rows now.)  Rows per block: 1,000 rows 0.50 / 0.38 / 0.33 / 0.29 ms with 512 / 256 /
 // 128 / 64.
 constexpr int kClusterRows = 12288, kClusterRowsPerBlock = 64;
 
@@ -902,7 +895,7 @@ int pcg_amg_grid_blocks() {
 
 // Largest cluster (a power of two) of the kernel on the current device.
 static int query_cluster_blocks() {
-    const void *fn = (const void *)k_pcg_amg<ClusterSync, 2>;
+    const void *fn = (const void *)k_pcg_amg<ClusterSync, 1>;
     const bool large = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     if (!large) cudaGetLastError();
     for (int k = large ? kClusterMax : 8; k > 1; k /= 2) {
@@ -952,7 +945,7 @@ int launch_pcg_amg(const PcgArgs &a, const AmgDev &amg, cudaStream_t st) {
         cfg.stream = st;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        return (int)cudaLaunchKernelExC(&cfg, (const void *)k_pcg_amg<ClusterSync, 2>, params);
+        return (int)cudaLaunchKernelExC(&cfg, (const void *)k_pcg_amg<ClusterSync, 1>, params);
     }
     int nb = pcg_amg_grid_blocks();
     // one row per thread where the blocks suffice; below one block per SM twice

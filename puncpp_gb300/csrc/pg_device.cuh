@@ -252,7 +252,7 @@ struct PcgArgs {
     double *p0;
     double *p1;
     double *Ap;
-    double *partials;             // [6][grid]
+    double *partials;             // [5][grid]
     double rtol, atol;
     int32_t max_iter;
     int32_t remove_mean;          // periodic: project b and x onto mean zero
