@@ -949,6 +949,25 @@ def combine_replicas(res, world):
     return out
 
 
+# What a printed line leaves out: the errors step by step and the prose. The
+# line of the default workload was 20,800 characters with them, 12,200 of them
+# the per-step errors, more than a log's tail keeps, and was lost with its start.
+LINE_WITHOUT = {"per_step_l2", "per_step_interior_l2", "per_step_max", "how", "what", "path", "sample", "timing",
+                "window", "algorithmic_bytes", "traffic_source", "traffic_unit", "stage_share", "stage_source",
+                "roofline_pcg", "poisson_form", "collected_current_equal_steps"}
+
+
+def line(res):
+    """The record as one JSON line of some 4,000 characters."""
+    def short(v):
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items() if k not in LINE_WITHOUT}
+        if isinstance(v, list):
+            return [short(x) for x in v]
+        return float("%.6g" % v) if isinstance(v, float) and abs(v) < 1e5 else v
+    return json.dumps(short(res), separators=(",", ":"))
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1, help="GPUs of the job (N > 1: one replica per rank under torchrun)")
@@ -988,6 +1007,7 @@ def main():
                     help="probe workloads: particle store slots per initial particle (the store grows if needed)")
     ap.add_argument("--runs", type=int, default=64, help="batch-R: runs in the batch (from the workload name)")
     ap.add_argument("--adjoint-particles", type=int, default=2_000_000, help="adjoint-N: particles of the run")
+    ap.add_argument("--details", default=None, help="file for the whole record, errors step by step included")
     args = ap.parse_args()
     kind = args.workload.split("-")[0]
     if kind not in ("config3", "probe", "langmuir", "batch", "adjoint"):
@@ -1033,7 +1053,7 @@ def main():
                             "particle_stages": r64["particle_stages"], "long_run": r64["long_run"],
                             "stage_ms_per_step": r64["stage_ms_per_step"], "tuning": r64["config"]["tuning"],
                             "amg_theta": r64["config"]["amg_theta"],
-                            "poisson": "the same AMG-preconditioned PCG as the mixed form (FP32 recurrence and "
+                            "poisson_form": "the same AMG-preconditioned PCG as the mixed form (FP32 recurrence and "
                                        "operators, FP64 solution, inner products and true-residual replacement, "
                                        "FP64 stopping test); the particle arithmetic is FP64"}
         # the full step shares the Poisson solve between the forms; the
@@ -1053,7 +1073,10 @@ def main():
     if rank == 0:
         if not args.no_cpu_baseline:
             res["cpu_baseline"] = cpu_baseline(args)
-        print(json.dumps(res))
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(res, f, indent=1)
+        print(line(res))
 
 
 if __name__ == "__main__":
