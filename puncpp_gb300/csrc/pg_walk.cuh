@@ -116,11 +116,11 @@ constexpr int kNearSteps = 256;
 // the only one whose four plane values are not positive, the one where the
 // long walk ends too.  Otherwise the long walk runs.
 template <bool NEAR, class T>
-__device__ __forceinline__ int walk_screened(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
-                                             CellRec &R, bool have_rec, float l[4]) {
+__device__ __forceinline__ int walk_loop(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
+                                         CellRec &R, bool have_rec, float l[4]) {
     const float xf = (float)x, yf = (float)y, zf = (float)z, ea = point_bound(m, xf, yf, zf);
     int cc = c;
-    bool near_walk = false, may_restart = NEAR && m.box != 0;
+    bool near_walk = false, may_restart = NEAR;
     for (int it = 0; it < max_steps; ++it) {
         float e[4];
         if (!have_rec) R = load_rec(m, cc);
@@ -156,6 +156,16 @@ __device__ __forceinline__ int walk_screened(const DevMesh &m, T x, T y, T z, in
         cc = next;
     }
     return kWalkFail;
+}
+
+// A mesh without a restart takes the loop without its tests: in one loop they
+// made the walk of Population::update in such meshes 10% slower (4M particles at
+// 48^3 cells, mixed form, 125 -> 138 us).
+template <bool NEAR, class T>
+__device__ __forceinline__ int walk_screened(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
+                                             CellRec &R, bool have_rec, float l[4]) {
+    return NEAR && m.box ? walk_loop<true>(m, x, y, z, c, max_steps, retests, R, have_rec, l)
+                         : walk_loop<false>(m, x, y, z, c, max_steps, retests, R, have_rec, l);
 }
 
 __device__ __forceinline__ int walk_mixed(const DevMesh &m, float x, float y, float z, int c, int max_steps,
