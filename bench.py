@@ -530,19 +530,20 @@ def amg_iteration_bytes(lay):
     bytes the engine reports (stored entries, padding excluded, times their
     stored size: f32 or binary16 value + 32- or 16-bit column; A_0 twice, for
     the PCG product and the level-0 smoother; every other cycle operator once)
-    plus the vectors, f32 except the f64 solution: 88 B per level-0 row (p, Ap,
-    z, r, t, x, D^-1 streams of the iteration's phases), 16 B per row of levels
-    1..L-1, 8 B per level-1 row (the up-sweep result)."""
+    plus the vectors, f32 except the f64 solution: 80 B per level-0 row (20 in
+    A p: z, p, Ap; 40 in the update: x, p, Ap, r, D^-1, s; 4 in the restriction: r;
+    16 in the prolongation: s, r, D^-1, z), 16 B per row of levels 1..L-1, 8 B per
+    level-1 row (the up-sweep result)."""
     lv = lay["levels"]
     if not lv:
         return 0, "no AMG levels"
     L = len(lv) - 1
-    b = lay["cycle_bytes"] + 88 * lv[0]["rows"]
+    b = lay["cycle_bytes"] + 80 * lv[0]["rows"]
     for l in range(1, L):
         b += 16 * lv[l]["rows"]
     b += 8 * lv[1]["rows"] if L >= 2 else 0
     return b, ("per iteration: operator bytes as stored (cycle_bytes: entries x stored size, A_0 twice) + "
-               "88*rows(0) + 16*rows(1..L-1) + 8*rows(1); operators re-read from L2 count each time")
+               "80*rows(0) + 16*rows(1..L-1) + 8*rows(1); operators re-read from L2 count each time")
 
 
 def ctypes_ms(lib, pop, a, b):

@@ -101,7 +101,9 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = N / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double sum4(const double *p, int step) { return (p[0] + p[step]) + (p[2 * step] + p[3 * step]); }
+__device__ __forceinline__ double sum4(const double *p, int step) {
+    return (p[0] + p[step]) + (p[2 * step] + p[3 * step]);
+}
 
 // The block's sum of v, for the total after the caller's barrier: stored to
 // part[blockIdx.x] in global memory, or in a cluster in every block's shared
@@ -482,7 +484,8 @@ struct Prolong {
         si = s[i]; ri = r[i]; di = __ldg(dinv + i);
         ea.load(A, ha.off(i), ha.width(), ha.h.y);
     }
-    __device__ __forceinline__ void first(const SpOp &A, const SpOp &S, const float *s, const float *r, const float *dinv, int i0, int i1) {
+    __device__ __forceinline__ void first(const SpOp &A, const SpOp &S, const float *s, const float *r,
+                                          const float *dinv, int i0, int i1) {
         if (!kAhead) return;
         ha.load(A, i0, i1);
         hs.load(S, i0, i1);
@@ -564,8 +567,8 @@ __device__ __forceinline__ int split_point(const SpOp &A, const SpOp &B, int nb)
 // SELL matrix; x read through L2, it is written inside the kernel) into r in
 // FP32 and, with s, omega D^-1 r into s; returns this thread's share of
 // ||b - A x||^2 and, with want_bb, adds its share of ||b||^2 to bb.
-__device__ __forceinline__ double true_residual(const PcgArgs &a, float *r, float *s, float om, bool want_bb, double &bb,
-                                             int i0, int i1, int gst) {
+__device__ __forceinline__ double true_residual(const PcgArgs &a, float *r, float *s, float om, bool want_bb,
+                                                double &bb, int i0, int i1, int gst) {
     double rr = 0.0;
     for (int i = i0; i < i1; i += gst) {
         double q = 0.0;
@@ -870,15 +873,16 @@ __global__ void __launch_bounds__(kPcgThreads, kBlocks) k_pcg_amg(const __grid_c
 
 // Systems of at most kClusterRows rows run on one cluster, as many blocks (a
 // power of two, at most 16) as leave kClusterRowsPerBlock rows to each: its
-// barrier is the hardware's (0.3 against 1.3 us of a cooperative grid, six
-// times an iteration) and its sums stay in shared memory, while its 16 SMs are
-// enough for so few rows.  Measured, solve on the grid -> on the cluster: 2,744
+// barrier is the hardware's (0.6 us after stores of all threads, 0.37 of it
+// their release, against 1.2 us of a cooperative grid, 1.4 with two blocks per
+// SM; six times an iteration) and its sums stay in shared memory, while its 16
+// SMs are enough for so few rows.  Measured, solve on the grid -> on the cluster: 2,744
 // rows 0.84 -> 0.45 ms, 9,260 0.49 -> 0.385, 13,824 0.467 -> 0.474 and, periodic, 0.64
 // -> 0.66, 39,298 0.61 -> 0.93, so the line lies between the second and the
 // third.  (With FP64 sums and the restriction in a phase of its own: 9,248 rows
 // 0.437 -> 0.354, 15,606 0.466 -> 0.426, 24,362 0.462 -> 0.515; the line could lie at
-// 17,000 rows now.)  Rows per block: 1,000 rows 0.50 / 0.38 / 0.33 / 0.29 ms with 512 / 256 /
-// 128 / 64.
+// 17,000 rows now.)  Rows per block: 1,000 rows 0.50 / 0.38 / 0.33 / 0.29 ms with
+// 512 / 256 / 128 / 64.
 constexpr int kClusterRows = 12288, kClusterRowsPerBlock = 64;
 
 int pcg_amg_grid_blocks() {

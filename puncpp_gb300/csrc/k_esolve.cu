@@ -21,7 +21,7 @@
 // residual's norm in FP64.
 //
 // What bounds it: the gathers and the barrier of each iteration; in FP64 also
-// the 45 FP64 operations of a row at 1/64 of the FP32 rate; in the form for
+// the 58 FP64 operations of a row at 1/64 of the FP32 rate; in the form for
 // larger systems (k_mass_cheb3), which reads the matrix each time, the chain of
 // loads of a row.  Measured (GB300, solve with rhs and packing), CG -> that form ->
 // rows in registers (k_mass_cheb3_reg): FP64 9,260 dofs 563 -> 266 -> 101 us, FP32
@@ -571,7 +571,8 @@ int solve(const EsolveArgs &e, T *buf, const T *sval, const T *dinv, cudaStream_
     const int units = (e.n + 31) / 32 * (3 / NC), sms = sm_count();
     if (units <= kRegThreads / 32 * sms) {
         const int nb = units < sms ? units : sms, warps = (units + nb - 1) / nb;
-        return (int)cudaLaunchCooperativeKernel((const void *)k_mass_cheb3_reg<T, NC>, dim3(nb), dim3(32 * warps), params, 0, st);
+        return (int)cudaLaunchCooperativeKernel((const void *)k_mass_cheb3_reg<T, NC>, dim3(nb), dim3(32 * warps),
+                                                params, 0, st);
     }
     int blocks = 0, threads = 0;
     launch_shape<T>(e.n, blocks, threads);

@@ -45,14 +45,15 @@ __device__ __forceinline__ bool inside_fp64(const DevMesh &m, double x, double y
 }
 
 // One pass over the particle slots doing any of push, move, walk and deposit.
-// Bound by the FP64 pipe (about 47 operations a particle, none contracted
-// where the reference's bits count).  The lanes of a warp take their 32 slots
-// together and meet again before and after the walk, whose lanes end in
-// different iterations: left to run on apart, 18 of 32 lanes were active in
-// an average instruction, and every FP64 operation of a part of a warp costs
-// as much as that of a whole one (53^3 cells, 1.5M particles: 224 -> 153 us, of
-// which 112 are the FP64 operations at full rate; the mixed form's pass, bound
-// by loads, does not change with it).
+// Bound by the FP64 pipe (47 operations a particle: Boris push 9, kinetic energy
+// 4, move 6, conversions for the walk 3, barycentric coordinates 21, deposit 4; 42
+// more with the CG1 field; none contracted but the kinetic energy's terms).  The
+// lanes of a warp take their 32 slots together and meet again before and after
+// the walk, whose lanes end in different iterations: left to run on apart, 18 of
+// 32 lanes were active in an average instruction, and every FP64 operation of a
+// part of a warp costs as much as that of a whole one (53^3 cells, 1.5M
+// particles: 224 -> 153 us, of which 112 are the FP64 operations at full rate; the
+// mixed form's pass, bound by loads, does not change with it).
 template <bool PUSH, bool HAS_B, bool ACCEL, bool MOVE, bool PERIODIC, bool WALK, bool DEPOSIT>
 __global__ void __launch_bounds__(512) k_particles(DevMesh m, DevParticles p, int64_t n_slots, PushParams pp,
                                                        MoveParams mp, int max_steps, const double *__restrict__ qsp,

@@ -96,8 +96,9 @@ __device__ __forceinline__ int near_cell(const DevMesh &m, float x, float y, flo
 // The point lies this many facet heights or more beyond some facet of the
 // first cell: a walk of about as many cells.  Periodic moves wrap a particle
 // to the other side of the box, which is a walk through every cell between,
-// and its warp waits for it (24^3 cells, 663k thermal electrons: the FP64 pass
-// 2.44 ms with long FP64 walks, 0.24 ms now).
+// and its warp waits for it (24^3 cells, 663k thermal electrons, CG1 field: the
+// FP64 pass 2.44 ms with long walks on FP64 planes, 0.19 ms with the restart,
+// the FP32 tests and the warp kept together).
 constexpr float kFarLambda = -6.0f;
 constexpr int kNearSteps = 256;
 
@@ -106,15 +107,16 @@ constexpr int kNearSteps = 256;
 // point (T: double or float).  One 64-byte record per cell visited instead of
 // 144 bytes, and no FP64 operation outside the bound (a plane test is six, at
 // 1/64 of the FP32 rate; the FP64 pass over 1.5M particles at 53^3 cells 525
-// us with them, 224 without, then 153 with the warp kept together).  R, have_rec: the first cell's record when the
-// caller has it; R and l are the last cell's on return.
+// us with them, 224 without, then 153 with the warp kept together).  R, have_rec:
+// the first cell's record when the caller has it; R and l are the last cell's on
+// return.
 //
 // NEAR: in a box without an inner wall (m.box; set only with a step limit that
 // no walk through such a mesh reaches) a walk that starts far from its point
-// starts again at a cell near it.  The result counts only if the
-// point lies inside its cell by more than the error bounds: that cell is then
-// the only one whose four plane values are not positive, the one where the
-// long walk ends too.  Otherwise the long walk runs.
+// starts again at a cell near it.  The result counts only if the point lies
+// inside its cell by more than the error bounds: that cell is then the only one
+// whose four plane values are not positive, the one where the long walk ends
+// too.  Otherwise the long walk runs.
 template <bool NEAR, class T>
 __device__ __forceinline__ int walk_loop(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
                                          CellRec &R, bool have_rec, float l[4]) {
