@@ -58,13 +58,13 @@ def workload_name(n_side, n_per):
 # particle pass per launch, the PCG per iteration at the AMG strength threshold
 # of the capture (scaled by this run's iterations per solve)
 PROFILED_TRAFFIC = {
-    ("probe-80", "k_pcg_amg", 0.0): (1.204e9 / 17, "profiles/k_pcg_amg_probe80_mixed.md: 987 MB read + 217 MB "
-                                                   "written per solve of 17 iterations"),
+    ("probe-80", "k_pcg_amg", 0.0): (1.127e9 / 17, "profiles/k_pcg_amg_forms.md: 987 MB read + 140 MB written per "
+                                                   "solve of 17 iterations"),
     ("probe-80", "k_mixed", None): (0.562e9, "profiles/k_mixed_probe80.md: 455 MB read + 106 MB written per launch"),
-    ("config3-120", "k_pcg_amg", 0.0): (10.99e9 / 20, "profiles/k_pcg_amg_config3_120.md (threshold 0): 9.73 GB "
-                                                      "read + 1.27 GB written per solve of 20 iterations"),
-    ("config3-120", "k_pcg_amg", 0.01): (10.463e9 / 17, "profiles/k_pcg_amg_config3_120.md (threshold 0.01): 9.30 GB "
-                                                        "read + 1.16 GB written per solve of 17 iterations"),
+    ("config3-120", "k_pcg_amg", 0.0): (10.48e9 / 20, "profiles/k_pcg_amg_config3_120.md (threshold 0): 9.43 GB "
+                                                      "read + 1.05 GB written per solve of 20 iterations"),
+    ("config3-120", "k_pcg_amg", 0.01): (9.939e9 / 17, "profiles/k_pcg_amg_config3_120.md (threshold 0.01): 9.00 GB "
+                                                       "read + 0.94 GB written per solve of 17 iterations"),
     ("config3-120", "k_mixed", None): (2.89e9, "profiles/k_mixed_config3_120.md: 2.30 GB read + 0.59 GB written per "
                                                "launch (untuned 256 x 4 launch configuration)"),
 }
