@@ -52,8 +52,7 @@ struct DevMesh {
     const float4 *cell_f = nullptr;   // [nc][4]
     float *E_f = nullptr;             // [nc][4] FP32 field (mixed form)
     // bound on the rounding of the FP64 tables in lambda (launch_float_tables)
-    // for points with coordinates up to 1 / lam_inv_range; beyond, it grows with
-    // the largest coordinate (point_bound)
+    // for points with coordinates up to 1 / lam_inv_range
     float lam_abs = 0.0f, lam_inv_range = 0.0f;
     // CG1 (vertex) field of the ESolver path: [ndof][4] (x, y, z, 0)
     const double *Ev = nullptr;

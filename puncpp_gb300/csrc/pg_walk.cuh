@@ -28,7 +28,7 @@ __device__ __forceinline__ double plane64(double c0, double c1, double c2, doubl
 // Relative bound on |FP32 affine value - exact value| in units of the sum of
 // the terms' magnitudes: one rounding per coefficient, coordinate and fmaf
 // (at most five), and slack.  The absolute part of the bound is the mesh's
-// (point_bound, the rounding of the FP64 tables).
+// (DevMesh::lam_abs, the rounding of the FP64 tables).
 constexpr float kPlaneEps = 8.0f * 5.9604645e-08f;   // 8 * 2^-24
 
 // Cell record of c: barycentric rows 0-2 in FP32 and the neighbours (int bits).
@@ -40,26 +40,17 @@ __device__ __forceinline__ CellRec load_rec(const DevMesh &m, int c) {
     return CellRec{__ldg(R), __ldg(R + 1), __ldg(R + 2), __ldg(R + 3)};
 }
 
-// The mesh's absolute error bound at a point: the tables' errors are affine in
-// its coordinates, so beyond the range that lam_abs holds for, the bound grows as
-// the largest of them.  (The relative bound does not cover that: a coefficient
-// that should be zero is 1e-17 in one FP64 table and zero in the other, and at
-// 1e12 box sizes the term is larger than the rounding of those that count.)
-__device__ __forceinline__ float point_bound(const DevMesh &m, float x, float y, float z) {
-    return m.lam_abs * fmaxf(1.0f, m.lam_inv_range * fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))));
-}
-
 // Barycentric coordinates of the FP32 point from a cell record's rows 0-2
 // (the fourth is 1 - l0 - l1 - l2) and bounds on their distance from the
 // FP64 planes' values over the heights, at the FP32 point and at any FP64
-// point that rounds to it (ea: point_bound).
-__device__ __forceinline__ void lambdas_f32(const CellRec &R, float ea, float x, float y, float z, float l[4],
+// point that rounds to it.
+__device__ __forceinline__ void lambdas_f32(const DevMesh &m, const CellRec &R, float x, float y, float z, float l[4],
                                             float e[4]) {
     const float4 r[3] = {R.r0, R.r1, R.r2};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         l[k] = fmaf(r[k].w, z, fmaf(r[k].z, y, fmaf(r[k].y, x, r[k].x)));
-        e[k] = fmaf(kPlaneEps, fabsf(r[k].x) + fabsf(r[k].y * x) + fabsf(r[k].z * y) + fabsf(r[k].w * z), ea);
+        e[k] = fmaf(kPlaneEps, fabsf(r[k].x) + fabsf(r[k].y * x) + fabsf(r[k].z * y) + fabsf(r[k].w * z), m.lam_abs);
     }
     l[3] = __fsub_rn(__fsub_rn(__fsub_rn(1.0f, l[0]), l[1]), l[2]);
     e[3] = e[0] + e[1] + e[2] + kPlaneEps * (1.0f + fabsf(l[0]) + fabsf(l[1]) + fabsf(l[2]));
@@ -120,14 +111,21 @@ constexpr int kNearSteps = 256;
 template <bool NEAR, class T>
 __device__ __forceinline__ int walk_loop(const DevMesh &m, T x, T y, T z, int c, int max_steps, int &retests,
                                          CellRec &R, bool have_rec, float l[4]) {
-    const float xf = (float)x, yf = (float)y, zf = (float)z, ea = point_bound(m, xf, yf, zf);
+    float xf = (float)x;
+    const float yf = (float)y, zf = (float)z;
+    // beyond the range of m.lam_abs (no cell holds such a point) every facet is
+    // tested in FP64: the tables' errors grow with the point's distance, and the
+    // relative bound does not cover them (a coefficient that should be zero is
+    // 1e-17 in one FP64 table and zero in the other: at 1e12 boxes the term is
+    // larger than the rounding of those that count)
+    if (!(m.lam_inv_range * fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf))) <= 1.0f)) xf = nanf("");
     int cc = c;
     bool near_walk = false, may_restart = NEAR;
     for (int it = 0; it < max_steps; ++it) {
         float e[4];
         if (!have_rec) R = load_rec(m, cc);
         have_rec = false;
-        lambdas_f32(R, ea, xf, yf, zf, l, e);
+        lambdas_f32(m, R, xf, yf, zf, l, e);
         if (NEAR && may_restart && fminf(fminf(l[0], l[1]), fminf(l[2], l[3])) < kFarLambda) {
             cc = near_cell(m, xf, yf, zf);
             near_walk = true;
