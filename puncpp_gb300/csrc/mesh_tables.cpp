@@ -462,45 +462,59 @@ int build_mesh(const pg_mesh_desc *d, double eps0, HostMesh &h) {
     return PG_OK;
 }
 
-// A plate of no thickness, a hole of any size and a second component all have
+// A plate of no thickness, a hole of any size and boxes side by side all have
 // facets without a neighbour inside the bounding box, so the facets are looked
-// at and not the volume alone.  The volume tells a box that is covered once.
+// at and not the volume alone.  With every such facet in a plane of the box the
+// cells around a point inside number the same everywhere in it; the volume says
+// that it is one, which also leaves no second component.
 int64_t box_span(const HostMesh &h) {
     double vol = 0.0, box = 1.0;
     for (double v : h.volume) vol += v;
     for (int j = 0; j < 3; ++j) box *= h.bbox_hi[j] - h.bbox_lo[j];
     if (!(std::fabs(vol - box) <= 1e-9 * box)) return 0;
+    int64_t corner[8] = {-1, -1, -1, -1, -1, -1, -1, -1};   // a cell at each corner of the box
     for (int64_t c = 0; c < h.nc; ++c)
         for (int f = 0; f < 4; ++f) {
             if (h.nbr[4 * c + f] >= 0) continue;
-            bool wall = false;
-            for (int j = 0; j < 3 && !wall; ++j) {
-                bool lo = true, hi = true;
-                for (int i = 0; i < 4; ++i) {
-                    if (i == f) continue;
+            bool lo[3] = {true, true, true}, hi[3] = {true, true, true};
+            for (int i = 0; i < 4; ++i) {
+                if (i == f) continue;
+                int k = 0, on = 0;
+                for (int j = 0; j < 3; ++j) {
                     const double x = h.coords[3 * h.cell_vertices[4 * c + i] + j];
-                    lo = lo && x == h.bbox_lo[j];
-                    hi = hi && x == h.bbox_hi[j];
+                    const bool l = x == h.bbox_lo[j], u = x == h.bbox_hi[j];
+                    lo[j] = lo[j] && l;
+                    hi[j] = hi[j] && u;
+                    on += l || u;
+                    k |= u ? 1 << j : 0;
                 }
-                wall = lo || hi;
+                if (on == 3 && corner[k] < 0) corner[k] = c;
             }
-            if (!wall) return 0;
+            if (!(lo[0] || lo[1] || lo[2] || hi[0] || hi[1] || hi[2])) return 0;
         }
-    // breadth first from cell 0
-    std::vector<char> seen(h.nc, 0);
-    std::vector<int32_t> front{0}, next;
-    seen[0] = 1;
-    int64_t reached = 0, span = -1;
-    for (; !front.empty(); front.swap(next), ++span) {
-        reached += (int64_t)front.size();
-        next.clear();
-        for (int32_t c : front)
-            for (int f = 0; f < 4; ++f) {
-                const int64_t o = h.nbr[4 * (int64_t)c + f];
-                if (o >= 0 && !seen[o]) { seen[o] = 1; next.push_back((int32_t)o); }
+    // relocate_fast from each corner to the middle of every other's cell
+    int64_t span = 1;
+    for (int a = 0; a < 8; ++a)
+        for (int b = 0; b < 8; ++b) {
+            if (corner[a] < 0 || corner[b] < 0) return 0;
+            double x[3] = {0.0, 0.0, 0.0};
+            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 3; ++j) x[j] += 0.25 * h.coords[3 * h.cell_vertices[4 * corner[b] + i] + j];
+            int64_t c = corner[a], steps = 0;
+            for (; steps <= h.nc; ++steps) {
+                int f = 0;
+                for (; f < 4; ++f) {
+                    const double *P = &h.planes[16 * c + 4 * f];
+                    if (P[0] + P[1] * x[0] + P[2] * x[1] + P[3] * x[2] > 0) break;
+                }
+                if (f == 4) break;
+                c = h.nbr[4 * c + f];
+                if (c < 0) return 0;
             }
-    }
-    return reached == h.nc ? std::max<int64_t>(1, span) : 0;
+            if (c != corner[b]) return 0;
+            span = std::max(span, steps);
+        }
+    return span;
 }
 
 }  // namespace pg

@@ -32,10 +32,10 @@ constexpr int kWalkFail = -2147483647;    // walk step limit reached
 // (box_span), which a walk through it does not reach, so that a walk that ends
 // with the limit's error does so with and without a restart.  In a box cut by
 // whole planes (Kuhn cells) each step of a walk crosses one of the planes between
-// its cell and its point, and none twice: it takes no more steps than lie
-// between two cells, at most two spans.  The rest is for cells of other
-// shapes.  (A walk that never ends, which cells cut against the Delaunay
-// condition allow, is an error without a restart and may find its cell with it.)
+// its cell and its point, and none twice: at most as many as lie between two
+// cells, under two spans.  The rest is for cells of other shapes.  (A walk that
+// never ends, which cells cut against the Delaunay condition allow, is an error
+// without a restart and may find its cell with it.)
 constexpr int kBoxWalkSpans = 8;
 
 struct DevMesh {

@@ -38,10 +38,9 @@ struct HostMesh {
 
 int build_mesh(const pg_mesh_desc *d, double eps0, HostMesh &h);
 
-// The number of facets between the first cell and the one furthest from it, at
-// least 1, if the mesh is a box without an inner wall: every facet without a
-// neighbour lies in a plane of the bounding box, the cells are connected and
-// their volumes add up to the box's.  Else 0.
+// The steps of the longest walk between two corners of the mesh, at least 1, if
+// it is a box without an inner wall: every facet without a neighbour lies in a
+// plane of the bounding box and the cells' volumes add up to the box's.  Else 0.
 int64_t box_span(const HostMesh &h);
 
 void set_error(const std::string &msg);

@@ -48,13 +48,17 @@ def test_boxes_with_walls_are_no_boxes(span):
 @pytest.mark.parametrize("n", [1, 2, 5, 11])
 def test_span_of_a_box(span, n):
     """The cells lie between planes x, y, z = k h and x-y, x-z, y-z = k h, and a
-    way from one to another crosses each plane between them: the largest number
-    from the cell 0 < z < y < x < h is found by counting."""
+    walk from one to another crosses each plane between them once: counted for
+    the first cell at each corner."""
     ma = meshgen.kuhn_box(n, -1.0, 1.0)
-    c = (ma.coords[ma.cells].mean(axis=1) + 1.0) * n / 2
-    f = np.stack([c[:, 0], c[:, 1], c[:, 2], c[:, 0] - c[:, 1], c[:, 0] - c[:, 2], c[:, 1] - c[:, 2]])
-    far = np.abs(np.floor(f) - np.floor(f[:, :1])).sum(axis=0).max()
-    assert span(ma) == max(1, far)
+    p = (ma.coords[ma.cells] + 1.0) * n / 2
+    first = {}
+    for k, v in zip(*np.nonzero(np.all((p == 0) | (p == n), axis=2))):
+        first.setdefault(tuple(p[k, v]), k)
+    c = p[sorted(first.values())].mean(axis=1)
+    f = np.floor(np.stack([c[:, 0], c[:, 1], c[:, 2], c[:, 0] - c[:, 1], c[:, 0] - c[:, 2], c[:, 1] - c[:, 2]]))
+    assert len(first) == 8
+    assert span(ma) == max(1, np.abs(f[:, :, None] - f[:, None, :]).sum(axis=0).max())
 
 
 def test_span_of_a_slender_box(span):
